@@ -25,7 +25,19 @@
 // integer pipes and decide exactly as the double compare does, NaN included.
 // ---------------------------------------------------------------------------
 #define FSG_D_INF_BITS 0x7ff0000000000000ULL
-FSG_DEV unsigned long long dbits(double m) { return (unsigned long long)__double_as_longlong(m); }
+// the bits of a double.  Through an opaque move on the device: from a plain
+// bitcast the compiler recognises these tests and turns them back into double
+// compares on the FP64 pipe (XR64 at 513 x 511 on the period-2562 nucleus: 37.9
+// -> 23.1 ms; FP64 on the seahorse view: 16.6 -> 14.7 ms)
+FSG_DEV unsigned long long dbits(double m) {
+#ifdef __CUDA_ARCH__
+    unsigned long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(m));
+    return b;
+#else
+    return (unsigned long long)__double_as_longlong(m);
+#endif
+}
 // m == 0. (+0 or -0)
 FSG_DEV bool d_is0(double m) { return (dbits(m) << 1) == 0ULL; }
 // inf or NaN
@@ -39,12 +51,12 @@ FSG_DEV bool d_abs_le(double a, double b) {
 // square (never -0): non-negative doubles order as their bit patterns read as
 // signed integers, and a NaN on either side (of either sign) decides false
 FSG_DEV bool d_sq_gt(double s, double t) {
-    const long long a = __double_as_longlong(s), b = __double_as_longlong(t);
+    const long long a = (long long)dbits(s), b = (long long)dbits(t);
     return a > b && (unsigned long long)a <= FSG_D_INF_BITS
            && (dbits(t) << 1) <= (FSG_D_INF_BITS << 1);
 }
 FSG_DEV bool d_sq_lt(double s, double t) {
-    const long long a = __double_as_longlong(s), b = __double_as_longlong(t);
+    const long long a = (long long)dbits(s), b = (long long)dbits(t);
     return a < b && (unsigned long long)a <= FSG_D_INF_BITS
            && (dbits(t) << 1) <= (FSG_D_INF_BITS << 1);
 }
@@ -170,7 +182,7 @@ FSG_DEV xc xc_zero() { return xc_make(0., 0., 0); }
 
 // numba_xr.py _frexp: rewrite the biased exponent to 1023, m in [1, 2)
 FSG_DEV double xr_frexp(double m, int &e) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(m);
+    unsigned long long b = dbits(m);
     e = (int)((b >> 52) & 0x7ff) - 0x3ff;
     return __longlong_as_double((long long)((b & 0x8000000000000000ULL) + (0x3ffULL << 52)
                                             + (b & 0xfffffffffffffULL)));
@@ -182,7 +194,7 @@ FSG_DEV double xr_norm_real(double m, int exp, int &eo) {
 }
 // numba_xr.py _exp2_shift: add to the biased exponent, clamped at 0
 FSG_DEV double xr_exp2_shift(double m, long long shift) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(m);
+    unsigned long long b = dbits(m);
     long long ex = (long long)((b >> 52) & 0x7ff) + shift;
     if (ex < 0) ex = 0;
     return __longlong_as_double((long long)((b & 0x8000000000000000ULL)
@@ -190,7 +202,7 @@ FSG_DEV double xr_exp2_shift(double m, long long shift) {
                                             + (b & 0xfffffffffffffULL)));
 }
 FSG_DEV bool xr_need_renorm_r(double m) {
-    long long d = (long long)(((unsigned long long)__double_as_longlong(m) >> 52) & 0x7ff) - 1023;
+    long long d = (long long)((dbits(m) >> 52) & 0x7ff) - 1023;
     return (d < 0 ? -d : d) > 100;
 }
 FSG_DEV bool xr_need_renorm_c(double2 m) { return xr_need_renorm_r(m.x) || xr_need_renorm_r(m.y); }
