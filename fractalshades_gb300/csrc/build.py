@@ -43,7 +43,7 @@ SOURCES = {
     "fsg_postproc.cu": ["-fmad=false"],
     "fsg_abi.cu": [],
 }
-HEADERS = ["fsg_num.cuh", "fsg_internal.cuh", "fsg_bs.cuh", "fsg_mn.cuh"]
+HEADERS = ["fsg_num.cuh", "fsg_internal.cuh", "fsg_bs.cuh", "fsg_mn.cuh", "fsg_soft.cuh"]
 
 
 def nvcc():

@@ -248,6 +248,7 @@ CalcDev make_calc(const fsg_calc *c) {
     d.logd = log(c->nexp ? (double)c->nexp : 2.);
     d.backshift = c->backshift;
     d.d2 = c->calc_d2zndc2;
+    fsg_calc_thresholds(d);
     return d;
 }
 
@@ -343,7 +344,8 @@ int launch_on(fsg_ctx *ctx, const LaunchRes &L, const fsg_calc *calc, const Tile
     W.budget = (unsigned long long)calc->iter_budget; W.used = L.used_dev;
     CalcDev C = make_calc(calc);
     // one persistent wave at the kernel's occupancy limit, or the tuned shape
-    const int block = calc->block > 0 ? calc->block : default_block(calc, perturb);
+    // (0: the standard loop's launcher chooses by the size)
+    const int block = calc->block > 0 || !perturb ? calc->block : default_block(calc, perturb);
     const int grid = calc->ctas_per_sm > 0 ? -calc->ctas_per_sm : 0;
     if (L.ev0 && seg.first && !seg.keep_time) CK(cudaEventRecord(L.ev0, s), "cudaEventRecord");
     if (!perturb) fsg_launch_std(W, C, grid, block, s);

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include "fsg_num.cuh"
 #include "fsg_mn.cuh"
+#include "fsg_soft.cuh"
 
 #define FSG_MAX_TILES_PER_LAUNCH 1024
 #define FSG_STG_COMPRESSED 3          // settings.py:40 BLA_compression
@@ -130,7 +131,22 @@ struct CalcDev {
     double logd;                               // log of the degree (potential)
     int backshift;                             // > 0: orbit point n - backshift
     int d2;                                    // standard loop: d2zndc2 in row 3
+    SqBound esc, stat;                         // M2, eps2 on exponents (fsg_soft.cuh)
 };
+
+inline void fsg_calc_thresholds(CalcDev &C) {
+    C.esc = fsg_sq_bound(C.M2);
+    C.stat = fsg_sq_bound(C.eps2);
+    if (C.eps2 == 0.) C.stat.hi = 0u;          // |z|^2 < 0: never
+}
+// |z|^2 > M^2 and |dz/dz|^2 < eps^2 as the loops decide them: from the
+// exponents on every step but a few of a pixel's last ones
+__device__ __forceinline__ bool fsg_escaped(const CalcDev &C, double2 z) {
+    return d_abs2_gt(z, C.M2, C.esc);
+}
+__device__ __forceinline__ bool fsg_stationary(const CalcDev &C, double2 d) {
+    return d_abs2_lt(d, C.eps2, C.stat);
+}
 
 // Work distribution of one launch: a device counter hands out pixel indices
 // of the concatenated tiles.
@@ -149,6 +165,18 @@ struct WorkDev {
     unsigned long long *used;        // iterations of the pixels finished so far
 };
 
+// Tile and position in it of pixel g of the concatenated tiles
+__device__ __forceinline__ void fsg_locate(const WorkDev &W, const long long *s_start, long long g,
+                                           int &t, long long &ip) {
+    int lo = 0, hi = W.ntiles - 1;
+    while (lo < hi) {
+        int mid = (lo + hi + 1) >> 1;
+        if (s_start[mid] <= g) lo = mid; else hi = mid - 1;
+    }
+    t = lo;
+    ip = g - s_start[lo];
+}
+
 // Claim the next pixel: returns false when the work is exhausted, or when
 // the pixels finished so far have used the launch's iteration budget (the
 // status word then reads 2; pixels already claimed run to their end, the
@@ -162,14 +190,38 @@ __device__ __forceinline__ bool fsg_claim(const WorkDev &W, const long long *s_s
     long long g = W.base + (long long)atomicAdd(W.counter, 1ULL);
     if (g >= W.total) return false;
     if (W.order) g = (long long)W.order[g];
-    int lo = 0, hi = W.ntiles - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (s_start[mid] <= (long long)g) lo = mid; else hi = mid - 1;
-    }
-    t = lo;
-    ip = g - s_start[lo];
+    fsg_locate(W, s_start, g, t, ip);
     return true;
+}
+
+// Claim pixels for a warp, one per lane (all 32 lanes call it together): 32, or
+// `want` (1 .. 32) once fewer than 64 per warp of the grid are left, so that no
+// warp holds pixels back while others have run dry.  `last` (warp-uniform,
+// 0 at first) keeps the position of the previous claim.  Returns the number
+// claimed, for lanes 0 .. n - 1; 0 when the work is exhausted, the budget is
+// used (as fsg_claim) or the launch was cancelled.
+__device__ __forceinline__ int fsg_claim_warp(const WorkDev &W, const long long *s_start, int want,
+                                              long long &last, int &t, long long &ip) {
+    const int lane = threadIdx.x & 31;
+    const long long left = W.total - W.base - last;
+    const int ask = left >= 64LL * gridDim.x * (blockDim.x >> 5) ? 32 : want;
+    long long g = 0;
+    if (lane == 0) {
+        if (*W.cancel) { *W.status = 1; g = -1; }
+        else if (W.budget && *(volatile unsigned long long *)W.used >= W.budget) {
+            *W.status = 2; g = -1;
+        } else g = (long long)atomicAdd(W.counter, (unsigned long long)ask);
+    }
+    g = __shfl_sync(0xffffffffu, g, 0);
+    if (g < 0 || g >= W.total - W.base) return 0;
+    last = g;
+    const int got = (int)min((long long)ask, W.total - W.base - g);
+    if (lane < got) {
+        g += W.base + lane;
+        if (W.order) g = (long long)W.order[g];
+        fsg_locate(W, s_start, g, t, ip);
+    }
+    return got;
 }
 
 // a finished pixel's iterations, counted against the launch's budget
