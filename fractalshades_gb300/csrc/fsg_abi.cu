@@ -342,6 +342,8 @@ int launch_on(fsg_ctx *ctx, const LaunchRes &L, const fsg_calc *calc, const Tile
     W.counter = L.counter_dev; W.stats = L.stats_dev;
     W.cancel = ctx->cancel_dev; W.status = L.status_dev;
     W.budget = (unsigned long long)calc->iter_budget; W.used = L.used_dev;
+    // (a segment of a streamed call must run the pixels of its own range)
+    W.blocked = perturb && !seg.order && seg.base == 0 && seg.end == tiles_pixels(tiles, ntiles);
     CalcDev C = make_calc(calc);
     // one persistent wave at the kernel's occupancy limit, or the tuned shape
     // (0: the standard loop's launcher chooses by the size)

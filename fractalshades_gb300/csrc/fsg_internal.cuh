@@ -163,6 +163,7 @@ struct WorkDev {
     int *status;                     // device status word (1 = interrupted, 2 = budget)
     unsigned long long budget;       // iteration budget of the launch (0: none)
     unsigned long long *used;        // iterations of the pixels finished so far
+    int blocked;                     // rectangles are claimed in blocks of 8 x 4 pixels
 };
 
 // Tile and position in it of pixel g of the concatenated tiles
@@ -175,6 +176,31 @@ __device__ __forceinline__ void fsg_locate(const WorkDev &W, const long long *s_
     }
     t = lo;
     ip = g - s_start[lo];
+}
+
+// The j-th pixel of an nx x ny rectangle taken in blocks of 8 x 4 (row by row
+// inside a block, blocks row by row, then what is left at the right and at the
+// bottom), as an index in row-major order.  The lanes of a warp claim together
+// and leave their pixels' loop together: a warp is held up by its longest pixel,
+// and counts differ less over 8 x 4 pixels than over 32 x 1 (FE32, seahorse view
+// 1024 x 1024: 4.85 -> 4.45 ms; 16 x 2: 4.6 ms; views without escapes pay 0.2 %).
+__device__ __forceinline__ long long fsg_block_pixel(int nx, int ny, long long j) {
+    const int bx = nx >> 3, by = ny >> 2;
+    const long long whole = (long long)bx * by * 32;
+    if (j < whole) {
+        const int b = (int)(j >> 5), l = (int)j & 31;
+        const int row = b / bx;
+        const int x = (b - row * bx) * 8 + (l & 7), y = row * 4 + (l >> 3);
+        return (long long)y * nx + x;
+    }
+    j -= whole;
+    const int rw = nx - bx * 8;
+    const long long right = (long long)rw * by * 4;
+    if (j < right) {
+        const int y = (int)(j / rw);
+        return (long long)y * nx + bx * 8 + (int)(j - (long long)y * rw);
+    }
+    return (long long)by * 4 * nx + (j - right);
 }
 
 // Claim the next pixel: returns false when the work is exhausted, or when
@@ -191,6 +217,10 @@ __device__ __forceinline__ bool fsg_claim(const WorkDev &W, const long long *s_s
     if (g >= W.total) return false;
     if (W.order) g = (long long)W.order[g];
     fsg_locate(W, s_start, g, t, ip);
+    if (W.blocked) {
+        const TileDev &T = W.tiles[t];
+        if (!T.pix) ip = fsg_block_pixel(T.nx, T.ny, ip);
+    }
     return true;
 }
 
@@ -233,6 +263,17 @@ __device__ __forceinline__ void fsg_account(const WorkDev &W, unsigned long long
 __device__ __forceinline__ bool fsg_cancelled(const WorkDev &W) {
     if (*W.cancel) { *W.status = 1; return true; }
     return false;
+}
+
+// Claim a pixel and poll the interruption flag: the flag is in host memory, a
+// microsecond away, and its read overlaps the claim's (a pixel claimed by an
+// interrupted launch stays unrun).
+__device__ __forceinline__ bool fsg_claim_poll(const WorkDev &W, const long long *s_start, int &t,
+                                               long long &ip) {
+    const int cancel = *W.cancel;
+    const bool got = fsg_claim(W, s_start, t, ip);
+    if (cancel) *W.status = 1;
+    return got && !cancel;
 }
 
 // shared memory of a kernel's tile offsets, sized at launch (dynamic)

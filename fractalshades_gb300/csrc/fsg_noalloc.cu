@@ -146,7 +146,7 @@ extern "C" int fsg_std_tiles_noalloc(const fsg_calc *calc, const fsg_tile *tiles
     W.order = nullptr;
     W.counter = &S->counter; W.stats = S->stats;
     W.cancel = &S->cancel; W.status = &S->status;
-    W.budget = 0ULL; W.used = nullptr;
+    W.budget = 0ULL; W.used = nullptr; W.blocked = 0;
     CalcDev C;
     C.max_iter = (int)calc->max_iter;
     C.M2 = calc->M_divergence * calc->M_divergence;

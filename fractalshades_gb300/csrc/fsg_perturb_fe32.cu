@@ -694,8 +694,7 @@ __global__ void __launch_bounds__(FE32_BLOCK, INTERIOR ? 6 : 7) k_perturb_m2_fe3
     fsg_load_starts(W, s_start);
     int t; long long ip;
     while (true) {
-        if (*W.cancel) { *W.status = 1; break; }
-        if (!fsg_claim(W, s_start, t, ip)) break;
+        if (!fsg_claim_poll(W, s_start, t, ip)) break;
         unsigned nfull = 0, nbla = 0, nreb = 0;
         const int n = pixel_fe32<INTERIOR>(W.tiles[t], C, ip, nfull, nbla, nreb);
         fsg_account(W, (unsigned long long)n);
