@@ -25,18 +25,11 @@ __device__ __forceinline__ bool bla_possible(const RefDev &R, int w) {
 
 // perturbation.py:2116-2170 ref_BLA_get on dz itself: returns the step (0 if
 // none) and the table index of the accepted entry.  The reference tests
-// abs(dz) < r, a hypot, against each candidate radius; abs_cmp (fsg_num.cuh)
-// gives the same answers from |dz|^2 on dz's own scale, and hypot(dz) is
-// computed (out of line) only where that leaves one open.
-// hypot(z) < r, with hypot(z) computed once per lookup (h < 0: not yet);
-// out of line, compare included (inlined, the FP64 form ran 1.4 % slower)
-static __device__ __noinline__ int bla_hypot_lt(double2 z, double r, double &h) {
-    if (h < 0.) h = hypot(z.x, z.y);
-    return h < r;
-}
-__device__ __forceinline__ int bla_lookup_z(const RefDev &R, double2 z, int w, int &ib) {
-    const AbsScaled a = abs_scaled(z);
-    double h = -1.;              // hypot(z), once needed
+// abs(dz) < r, a hypot, against each candidate radius; mag_lt (fsg_soft.cuh)
+// decides all but about one in 10^5 from upper words, without FP64.
+// The search of ref_BLA_get with `lt(r)` for abs(dz) < r: the step and its index
+template <class LT>
+__device__ __forceinline__ int bla_search(const RefDev &R, int w, int &ib, LT lt) {
     int it = w >> FSG_STG_COMPRESSED;
     int stages = FSG_STG_COMPRESSED;
     for (int st = FSG_STG_COMPRESSED; st < R.stages; st++) {
@@ -49,12 +42,38 @@ __device__ __forceinline__ int bla_lookup_z(const RefDev &R, double2 z, int w, i
         const int step = 1 << stg;
         if (step >= invalid_step) continue;
         const int idx = 2 * (w >> FSG_STG_COMPRESSED) + ((1 << (stg - FSG_STG_COMPRESSED)) - 1);
-        const double r = __ldg(&R.rbla[idx]);
-        int lt = abs_cmp(a, r);
-        if (lt < 0) lt = bla_hypot_lt(z, r, h);
-        if (lt) { ib = idx; return step; }
+        if (lt(__ldg(&R.rbla[idx]))) { ib = idx; return step; }
     }
     return 0;
+}
+// |z| < r where upper words leave it open: abs_cmp, then hypot (a: |z|^2 on z's own
+// scale, h: hypot(z), each once per lookup)
+struct BLAExact { AbsScaled a; double h; bool has; };
+static __device__ __noinline__ int bla_exact_lt(double2 z, double r, BLAExact &x) {
+    if (!x.has) { x.a = abs_scaled(z); x.h = -1.; x.has = true; }
+    const int lt = abs_cmp(x.a, r);
+    if (lt >= 0) return lt;
+    if (x.h < 0.) x.h = hypot(z.x, z.y);
+    return x.h < r;
+}
+__device__ __forceinline__ int bla_lookup_z(const RefDev &R, double2 z, int w, int &ib) {
+    const MagF a = mag_of(z, 0);
+    BLAExact x;
+    x.has = false;
+    return bla_search(R, w, ib, [&](double r) {
+        const int lt = mag_lt(a, r);
+        return lt >= 0 ? lt : bla_exact_lt(z, r, x);
+    });
+}
+// the same for dz = z, an Xrange value whose standard value is compared
+__device__ __forceinline__ int bla_lookup_x(const RefDev &R, xc z, int w, int &ib) {
+    const MagF a = mag_of(xm(z), z.e);
+    BLAExact x;
+    x.has = false;
+    return bla_search(R, w, ib, [&](double r) {
+        const int lt = mag_lt(a, r);
+        return lt >= 0 ? lt : bla_exact_lt(xr_to_std(z), r, x);
+    });
 }
 
 // ---------------------------------------------------------------------------

@@ -229,6 +229,280 @@ __device__ __forceinline__ void pixel_m2(const TileDev &T, const CalcDev &C, lon
     itsum += (unsigned long long)n;
 }
 
+// Whether dz = z 2^e is below half an ulp of both parts of the orbit value Z (55
+// binary orders): Z + dz is then Z and dz + 2 Z is 2 Z, part by part.  False
+// where a part of Z is 0 or subnormal (values held in the Xrange side table
+// among them).
+__device__ __forceinline__ bool dz_below(double2 Z, double2 z, int e) {
+    const int lo = d_field_min(Z);
+    return lo > 0 && lo - d_field_max(z) - e >= 56;
+}
+
+// The power-2 loop, both delta forms.  The reference's operations with their
+// bits, arranged for GB300's pipes (an FP64 warp instruction holds its pipe for
+// 64 clocks and more, of which a step had 31): products on the integer pipes
+// (fsg_soft.cuh), sums left out where an operand is below half an ulp of the
+// other, the escape test and the BLA radii on upper words.  XR: every value is a
+// mantissa and an exponent of its own frame; the bits of a value do not depend
+// on the frame, so the frames of this loop differ from the reference's lazily
+// normalised ones (frame_add).  Whatever leaves the ranges those forms need
+// takes the reference's step, operation by operation.
+template <bool XR>
+__device__ __forceinline__ void pixel_m2_fast(const TileDev &T, const CalcDev &C, long long ip,
+                                              unsigned long long &nfull, unsigned long long &nbla,
+                                              unsigned long long &nreb, unsigned long long &itsum) {
+    const RefDev &R = *T.ref;
+    const long long np = (long long)T.nx * T.ny;
+    const bool dzndz_on = C.interior, dzndc_on = C.calc_dzndc;
+    const int order = R.order, div_iter = R.div_iter, w_wrapped = R.len;
+    // perturbation.py:2214-2230 ref_path_c_from_pix, 2666-2672 lin_proj_impl
+    const double2 pp = fsg_pixel(T, ip);
+    const double x1 = T.lin[0] * pp.x + T.lin[1] * pp.y;
+    const double y1 = T.lin[2] * pp.x + T.lin[3] * pp.y;
+    xf dxr; dxr.m = T.dx_m; dxr.e = T.dx_e;
+    const xc c_xr = xr_add(xf_mul_c(dxr, cx(x1, y1)), xc_make(T.drift_re, T.drift_im, T.drift_e));
+    const double2 c = XR ? xm(c_xr) : xr_to_std(c_xr);
+    const int ce = XR ? c_xr.e : 0;
+
+    // dz, dz/dc, dz/dz as mantissa and exponent (FP64: exponent 0 throughout);
+    // numba_initialize :1055-1060 (the per-tile Xrange dzndz carry-over of the
+    // reference is erased by the first full step, so it starts at zero here)
+    xc z = xc_zero(), v = xc_zero(), q = xc_zero();
+    int w = 0, n = 0; signed char stop = -1;
+    bool nullify = false, dyn = true;
+    const xc xzero = xc_zero();
+    double2 ZZ = cx(0., 0.);           // FP64: Z_w + dz of the last test,
+    bool has_ZZ = false;               // when the loop came straight from it
+
+    auto deriv_c = [&](int i) {        // dZndc_i
+        return XR ? ldx(R.dZndc_xm, R.dZndc_xe, i)
+                  : xc_make(__ldg(&R.dZndc[i]).x, __ldg(&R.dZndc[i]).y, 0);
+    };
+    auto deriv_z = [&](int i) {        // dZndz_i
+        return XR ? ldx(R.dZndz_xm, R.dZndz_xe, i)
+                  : xc_make(__ldg(&R.dZndz[i]).x, __ldg(&R.dZndz[i]).y, 0);
+    };
+    // in the ranges of the integer products: XR frames keep parts near 1, FP64
+    // parts have any size
+    auto ok2 = [&](double2 a, double2 b) { return XR ? dfac_ok(a) & dfac_ok(b) : cfac_ok<false>(a, b); };
+    // 2 (S d + D dz) by the integer products: S (exponent eS) and dz with their
+    // factors; dyn: D = 0, and S d stays as it is
+    auto deriv_step = [&](double2 S, int eS, const cfac &fS, const cfac &fz, xc d, xc D, bool dyn, bool &ok) {
+        ok = ok2(S, xm(d));
+        const double2 a = cfac_mul(fS, cfac_of(xm(d)), ok);
+        xc t = xc_make(a.x, a.y, eS + d.e);
+        if (!dyn) {
+            ok &= XR ? dfac_ok(xm(z)) & dfac_ok0(D.re) & dfac_ok0(D.im) : cfac_ok<true>(xm(D), xm(z));
+            const double2 b = cfac_mul0(cfac_of0(xm(D)), fz, ok);
+            if (XR) t = frame_add(a, eS + d.e, b, D.e + z.e, ok);
+            else { t.re += b.x; t.im += b.y; }
+        }
+        if (XR) {
+            t.e += 1;
+            frame_renorm(t, ok);
+        } else {
+            const double2 u = rmul2(xm(t));
+            t = xc_make(u.x, u.y, 0);
+        }
+        return t;
+    };
+
+    for (;;) {
+        // BLA step :1121-1154
+        if (C.bla && R.bla_len > 0 && (w & 7) == 0 && bla_possible(R, w)) {
+            int ib;
+            const int step = XR ? bla_lookup_x(R, z, w, ib) : bla_lookup_z(R, xm(z), w, ib);
+            if (step != 0) {
+                const double2 A = __ldg(&R.Mbla[2 * ib]), B = __ldg(&R.Mbla[2 * ib + 1]);
+                const cfac fA = cfac_of(A);
+                // A d
+                auto deriv_bla = [&](xc d) {
+                    bool ok = ok2(A, xm(d));
+                    const double2 t = cfac_mul(fA, cfac_of(xm(d)), ok);
+                    xc r = xc_make(t.x, t.y, d.e);
+                    if (XR) {
+                        frame_renorm(r, ok);
+                        if (!ok) r = xr_mul_s(A, d);
+                    } else if (!ok) {
+                        const double2 u = cmul(A, xm(d));
+                        r = xc_make(u.x, u.y, 0);
+                    }
+                    return r;
+                };
+                bool ok = ok2(A, xm(z)) & ok2(B, c);
+                const double2 a = cfac_mul(fA, cfac_of(xm(z)), ok), b = cfac_mul(cfac_of(B), cfac_of(c), ok);
+                xc nz;
+                if (XR) { nz = frame_add(a, z.e, b, ce, ok); frame_renorm(nz, ok); }
+                else { const double2 t = cadd(a, b); nz = xc_make(t.x, t.y, 0); }
+                if (!ok) {
+                    if (XR) {
+                        nz = xr_add(xr_mul_s(A, z), xr_mul_s(B, c_xr));
+                    } else {
+                        const double2 t = cadd(cmul(A, xm(z)), cmul(B, c));
+                        nz = xc_make(t.x, t.y, 0);
+                    }
+                }
+                z = nz;
+                if (dzndc_on) v = deriv_bla(v);
+                if (dzndz_on) q = deriv_bla(q);
+                n += step;
+                w += step;
+                if (w >= order) w = w % order;
+                has_ZZ = false;
+                nbla++;
+                continue;
+            }
+        }
+        // full perturbation step :1158-1214
+        n += 1;
+        nfull++;
+        const double2 Z = __ldg(&R.Zn[w]);
+        {
+            // S = Z + dz and T2 = dz + 2 Z (exponent e2): Z and 2 Z where dz is
+            // below half an ulp of Z, dz where Z is 0 (the critical point, once
+            // per period)
+            const bool below = dz_below(Z, xm(z), z.e);
+            const bool zero = XR && d_is0(Z.x) && d_is0(Z.y) && !(R.n_xr && __ldg(&R.xr_slot[w]) >= 0);
+            double2 S = Z, T2;
+            int e2 = 0;
+            if (XR) {
+                if (zero) { S = xm(z); e2 = z.e; }
+            } else if (!below) {
+                if (has_ZZ) S = ZZ; else S = cadd(Z, xm(z));
+            }
+            T2 = S;
+            if (!XR && !below) T2 = cadd(xm(z), rmul2(Z));
+            const bool in = !XR | below | zero;
+            const cfac fS = cfac_of(S), fz = cfac_of(xm(z));
+            cfac f2 = fS;
+            if (!XR && !below) f2 = cfac_of(T2);
+            else if (!zero) { f2.x.s += 0x00100000u; f2.y.s += 0x00100000u; }
+            xc nv = v, nq = q, nz;
+            bool okz = in & ok2(T2, xm(z)), okv = true, okq = true;
+            // (a derivative that is not asked for has no table to read)
+            if (dzndc_on) {
+                nv = deriv_step(S, e2, fS, fz, v, deriv_c(w), dyn, okv);
+                okv &= in;
+            }
+            if (dzndz_on) {
+                nq = deriv_step(S, e2, fS, fz, q, deriv_z(nullify ? 0 : w), false, okq);
+                okq &= in;
+            }
+            const double2 p = cfac_mul(fz, f2, okz);
+            if (XR) { nz = frame_add(p, e2 + z.e, c, ce, okz); frame_renorm(nz, okz); }
+            else { const double2 t = cadd(p, c); nz = xc_make(t.x, t.y, 0); }
+            // what is left open: the reference's operations
+            if (!(okz & okv & okq)) {
+                if (XR) {
+                    const int slot = R.n_xr ? __ldg(&R.xr_slot[w]) : -1;
+                    const xc Zx = (slot >= 0) ? ldx(R.xr_m, R.xr_e, slot) : xr_from(Z);
+                    const xc S2 = xr_add(Zx, z);
+                    if (!okv) nv = xr_mul_2(xr_add(xs_mul(S2, v), dyn ? xr_mul(xzero, z) : xs_mul(deriv_c(w), z)));
+                    if (!okq) nq = xr_mul_2(xr_add(xs_mul(S2, q), xs_mul(deriv_z(nullify ? 0 : w), z)));
+                    if (!okz) nz = xr_add(xs_mul(z, xr_add(z, xr_mul_2(Zx))), c_xr);
+                } else {
+                    if (!okv) {
+                        const double2 D = dyn ? cx(0., 0.) : xm(deriv_c(w));
+                        const double2 t = rmul2(cadd(cmul(S, xm(v)), cmul(D, xm(z))));
+                        nv = xc_make(t.x, t.y, 0);
+                    }
+                    if (!okq) {
+                        const double2 t = rmul2(cadd(cmul(S, xm(q)), cmul(xm(deriv_z(nullify ? 0 : w)), xm(z))));
+                        nq = xc_make(t.x, t.y, 0);
+                    }
+                    if (!okz) {
+                        const double2 t = cadd(cmul(xm(z), below ? rmul2(Z) : T2), c);
+                        nz = xc_make(t.x, t.y, 0);
+                    }
+                }
+            }
+            z = nz; v = nv; q = nq;
+        }
+        w += 1;
+        if (w >= order) w = w % order;
+        has_ZZ = false;
+        // max_iter :1218-1220
+        if (n >= C.max_iter) { stop = 0; break; }
+        // interior detection :1224-1246
+        if (dzndz_on) {
+            const xc D = deriv_z(nullify ? 0 : ((n == order) ? w_wrapped : w));
+            bool stat;
+            if (XR) stat = xf_sq_lt_s(xr_abs2(xr_add(q, D)), C.eps2);
+            else stat = fsg_stationary(C, cadd(xm(q), xm(D)));
+            if (stat) { stop = 2; break; }
+        }
+        const double2 Zn = __ldg(&R.Zn[w]);
+        // dz below half an ulp of Z_w: Z_w + dz = Z_w, and |Z_w + dz| <= |dz| holds
+        // in neither part
+        if (w < div_iter - 1 && dz_below(Zn, xm(z), z.e)) {
+            if (fsg_escaped(C, Zn)) { stop = 1; break; }
+            dyn = false;
+            ZZ = Zn;
+            has_ZZ = true;
+            continue;
+        }
+        // divergence :1252-1279
+        const double2 zn = XR ? xr_to_std(z) : xm(z);
+        ZZ = cadd(zn, Zn);
+        if (fsg_escaped(C, ZZ)) { stop = 1; break; }
+        // rebase when the reference diverges :1283-1313, dynamic rebase
+        // :1317-1372 (componentwise test, in the Xrange branch confirmed on the
+        // extended values)
+        bool rebase = w >= div_iter - 1;
+        xc nz = XR ? xr_from(ZZ) : xc_make(ZZ.x, ZZ.y, 0);
+        if (!rebase) {
+            dyn = d_abs_le(ZZ.x, zn.x) && d_abs_le(ZZ.y, zn.y);
+            has_ZZ = !XR;
+            rebase = dyn;
+            if (XR && dyn) {
+                const int slot = R.n_xr ? __ldg(&R.xr_slot[w]) : -1;
+                nz = (slot >= 0) ? xr_add(z, ldx(R.xr_m, R.xr_e, slot)) : xr_add_s(z, Zn);
+                rebase = xf_le(xr_abs2(nz), xr_abs2(z));
+            }
+        }
+        if (rebase) {
+            z = nz;
+            if (dzndc_on) v = XR ? xr_add(v, deriv_c(w)) : xc_make(v.re + deriv_c(w).re, v.im + deriv_c(w).im, 0);
+            if (dzndz_on) {
+                if (!nullify) {
+                    const xc D = deriv_z((n == order) ? w_wrapped : w);
+                    q = XR ? xr_add(q, D) : xc_make(q.re + D.re, q.im + D.im, 0);
+                }
+                nullify = true;
+            }
+            w = 0; nreb++;
+            has_ZZ = false;
+        }
+    }
+    // end of iterations :1375-1385
+    // dzndc in the tile's unit: the reference's scale times 2^dzs
+    const double2 zn = cadd(XR ? xr_to_std(z) : xm(z), __ldg(&R.Zn[w]));
+    double2 dzndc = cx(0., 0.), dzndz = cx(0., 0.);
+    if (dzndc_on) {
+        if (XR) {
+            xc t = xr_add(v, deriv_c(w));
+            t.e += T.dzs;
+            dzndc = xr_to_std(t);
+        } else {
+            dzndc = cadd(xm(v), xm(deriv_c(w)));
+            if (T.dzs != 0) dzndc = cx(ldexp_d(dzndc.x, T.dzs), ldexp_d(dzndc.y, T.dzs));
+        }
+    }
+    // (the Xrange branch never writes back Z[dzndz])
+    if (!XR) dzndz = xm(q);
+    double2 *Zo = (double2 *)T.Z;
+    Zo[ip] = zn;
+    if (dzndz_on) Zo[T.i_dzndz * np + ip] = dzndz;
+    // Expmap: derivatives times exp(Re(ht pix) + h_moy) (perturbation.py:1387-1388)
+    if (dzndc_on && T.proj) dzndc = rmul(fsg_dzndc_modifier(T, ip), dzndc);
+    if (dzndc_on) Zo[T.i_dzndc * np + ip] = dzndc;
+    if (T.U) T.U[ip] = w;
+    T.stop_iter[ip] = n;
+    T.stop_reason[ip] = stop;
+    fsg_epilogue(T, C, ip, zn, hypot(dzndc.x, dzndc.y), n);
+    itsum += (unsigned long long)n;
+}
+
 template <bool XR, bool MN, bool ORB>
 __global__ void __launch_bounds__(256) k_perturb_m2(WorkDev W, CalcDev C) {
     extern __shared__ long long s_start[];          // [W.ntiles + 1], sized at launch
@@ -238,7 +512,10 @@ __global__ void __launch_bounds__(256) k_perturb_m2(WorkDev W, CalcDev C) {
     while (true) {
         if (!fsg_claim_poll(W, s_start, t, ip)) break;
         const unsigned long long before = itsum;
-        pixel_m2<XR, MN, ORB>(W.tiles[t], C, ip, nfull, nbla, nreb, itsum);
+        if constexpr (MN || ORB)
+            pixel_m2<XR, MN, ORB>(W.tiles[t], C, ip, nfull, nbla, nreb, itsum);
+        else
+            pixel_m2_fast<XR>(W.tiles[t], C, ip, nfull, nbla, nreb, itsum);
         fsg_account(W, itsum - before);
     }
     fsg_flush_stats(W, itsum, nfull, nbla, nreb);

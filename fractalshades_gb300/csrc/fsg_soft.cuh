@@ -105,11 +105,134 @@ FSG_DEV double2 cfac_mul(const cfac &a, const cfac &b, bool &ok) {
     return cx(dfac_mul(a.x, b.x, ok) - dfac_mul(a.y, b.y, ok),
               dfac_mul(a.x, b.y, ok) + dfac_mul(a.y, b.x, ok));
 }
+// the same with zero parts allowed in a (its factors from dfac_of0)
+FSG_DEV cfac cfac_of0(double2 z) {
+    cfac f;
+    f.x = dfac_of0(z.x);
+    f.y = dfac_of0(z.y);
+    return f;
+}
+FSG_DEV double2 cfac_mul0(const cfac &a, const cfac &b, bool &ok) {
+    return cx(dfac_mul0(a.x, b.x, ok) - dfac_mul0(a.y, b.y, ok),
+              dfac_mul0(a.x, b.y, ok) + dfac_mul0(a.y, b.x, ok));
+}
 // csq: the cross product on the exponent of 2 x y
 FSG_DEV double2 cfac_sq(const cfac &a, bool &ok) {
     dfac x2 = a.x;
     x2.s += 0x00100000u;
     return cx(dfac_mul(a.x, a.x, ok) - dfac_mul(a.y, a.y, ok), dfac_mul(x2, a.y, ok));
+}
+
+// Whether the four products of a and b are normal, for parts of any normal size
+// (dfac_ok instead bounds each part).  Without `zeros` a zero part refuses; with
+// it, zero parts of a are left aside (dfac_of0).
+template <bool ZEROS>
+FSG_DEV bool cfac_ok(double2 a, double2 b) {
+    unsigned ax = d_hi(a.x) & 0x7ff00000u, ay = d_hi(a.y) & 0x7ff00000u;
+    const unsigned bx = d_hi(b.x) & 0x7ff00000u, by = d_hi(b.y) & 0x7ff00000u;
+    if (ZEROS) {
+        if (d_is0(a.x)) ax = ay;
+        if (d_is0(a.y)) ay = ax;
+    }
+    const unsigned la = min(ax, ay), ha = max(ax, ay), lb = min(bx, by), hb = max(bx, by);
+    return (min(la, lb) != 0u) & (max(ha, hb) != 0x7ff00000u) & (la + lb >= 1025u << 20)
+           & (ha + hb <= 3068u << 20);
+}
+
+// cmul, by the integer products where they can be (out of line elsewhere)
+static __device__ __noinline__ double2 cmul_full(double2 a, double2 b) { return cmul(a, b); }
+FSG_DEV double2 cmul_soft(double2 a, double2 b) {
+    bool ok = dfac_ok(a) & dfac_ok(b);
+    double2 r = cfac_mul(cfac_of(a), cfac_of(b), ok);
+    if (!ok) r = cmul_full(a, b);
+    return r;
+}
+
+// ---------------------------------------------------------------------------
+// Values m 2^e (xc): sums of two on one frame.  A sum of doubles rounds the same
+// on any power of two, so the value of p 2^ep + q 2^eq does not depend on the
+// frame it is taken on, while nothing leaves the normal range: the bits are
+// those of the reference's co-exponent sum.
+// ---------------------------------------------------------------------------
+FSG_DEV int d_field(double x) { return (int)(d_hi(x) >> 20 & 0x7ffu); }      // biased exponent
+// x 2^d for a normal x whose result is normal, 0 for 0
+FSG_DEV double d_shift(double x, int d) {
+    const int hi = (int)d_hi(x) + (d_is0(x) ? 0 : d << 20);
+    return __hiloint2double(hi, (int)d_lo(x));
+}
+// r = p 2^ep + q 2^eq, part by part.  A part 55 or more binary orders below the
+// other's leaves it as it is; where that holds for both parts there is no sum to
+// take.  ok is cleared where q does not fit p's frame.
+FSG_DEV xc frame_add(double2 p, int ep, double2 q, int eq, bool &ok) {
+    const int d = eq - ep;
+    const int px = d_field(p.x), py = d_field(p.y), qx = d_field(q.x), qy = d_field(q.y);
+    const int gx = px - qx - d, gy = py - qy - d;
+    if (min(gx, gy) >= 55 && min(px, py) > 0) return xc_make(p.x, p.y, ep);
+    if (max(gx, gy) <= -55 && min(qx, qy) > 0) return xc_make(q.x, q.y, eq);
+    ok &= ((unsigned)(qx + d - 1) < 2045u) | d_is0(q.x);
+    ok &= ((unsigned)(qy + d - 1) < 2045u) | d_is0(q.y);
+    return xc_make(p.x + d_shift(q.x, d), p.y + d_shift(q.y, d), ep);
+}
+// the larger part's exponent field (0 for zero and subnormal parts)
+FSG_DEV int d_field_max(double2 z) { return max(d_field(z.x), d_field(z.y)); }
+FSG_DEV int d_field_min(double2 z) { return min(d_field(z.x), d_field(z.y)); }
+// back to a frame with the larger part in 2^+-100 (one shift for both parts);
+// ok is cleared where the smaller part would leave the normal range
+FSG_DEV void frame_renorm(xc &a, bool &ok) {
+    const int k = d_field_max(xm(a)) - 1023;
+    if ((unsigned)(k + 100) <= 200u) return;
+    ok &= (d_field_min(xm(a)) - k >= 1) | d_is0(a.re) | d_is0(a.im);
+    ok &= k > -1023;                                    // not 0 (nor subnormal)
+    a.re = d_shift(a.re, -k);
+    a.im = d_shift(a.im, -k);
+    a.e += k;
+}
+
+// xr_mul and xr_mul_s by the integer products
+FSG_DEV xc xs_mul(xc a, xc b) {
+    double2 m = cmul_soft(xm(a), xm(b));
+    int e = (int)((unsigned)a.e + (unsigned)b.e);
+    if (xr_need_renorm_c(m)) return xr_normalize_c(m, e);
+    return xc_make(m.x, m.y, e);
+}
+FSG_DEV xc xs_mul_s(double2 s, xc b) {
+    double2 m = cmul_soft(s, xm(b));
+    if (xr_need_renorm_c(m)) return xr_normalize_c(m, b.e);
+    return xc_make(m.x, m.y, b.e);
+}
+
+// ---------------------------------------------------------------------------
+// |z| < r as hypot(z) < r decides it, from upper words: |z|^2 = q 2^2e with q in
+// [1, 8) known to a part in 2^18 (mag_of: the words as floats, cut to 20 bits, on
+// the larger part's exponent), against r^2 on the same exponent.  -1: too close,
+// or out of the normal range (abs_cmp and hypot decide, fsg_num.cuh).
+// ---------------------------------------------------------------------------
+struct MagF { float q; int e; bool ok; };
+FSG_DEV MagF mag_of(double2 z, int ze) {
+    const unsigned hx = d_hi(z.x) & 0x7fffffffu, hy = d_hi(z.y) & 0x7fffffffu, m = max(hx, hy);
+    const unsigned base = (m & 0x7ff00000u) - (127u << 20);
+    const float x = __int_as_float(max((int)(hx - base), 0) << 3);
+    const float y = __int_as_float(max((int)(hy - base), 0) << 3);
+    MagF a;
+    a.q = x * x + y * y;
+    a.e = (int)(m >> 20) - 1023 + ze;
+    a.ok = m >= 0x00100000u && m < 0x7ff00000u;
+    return a;
+}
+FSG_DEV int mag_lt(const MagF &a, double r) {
+    const unsigned h = d_hi(r);
+    if (d_is0(r)) return 0;                               // never below 0
+    if (!a.ok || h < 0x00100000u || h >= 0x7ff00000u) return -1;
+    const int d = (int)(h >> 20) - 1023 - a.e;
+    if (d >= 3) return 1;                                 // |z| < 2^(e + 1.5)
+    // (near the end of the doubles' range the loops compare the rounded value)
+    if (a.e < -1000) return -1;
+    if (d <= -2) return 0;                                // r < 2^(e - 1)
+    const float f = __int_as_float((int)((h & 0x000fffffu) << 3 | (unsigned)(d + 127) << 23));
+    const float f2 = f * f;
+    if (a.q * (1.f + 0x1p-17f) < f2) return 1;
+    if (a.q > f2 * (1.f + 0x1p-17f)) return 0;
+    return -1;
 }
 
 // ---------------------------------------------------------------------------

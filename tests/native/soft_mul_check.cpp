@@ -12,6 +12,9 @@
 #include <random>
 static inline long long __double_as_longlong(double d) { long long x; memcpy(&x, &d, 8); return x; }
 static inline double __longlong_as_double(long long x) { double d; memcpy(&d, &x, 8); return d; }
+static inline double __hiloint2double(int hi, int lo) {
+    return __longlong_as_double((long long)((unsigned long long)(unsigned)hi << 32 | (unsigned)lo));
+}
 static inline int __float_as_int(float f) { int x; memcpy(&x, &f, 4); return x; }
 static inline float __int_as_float(int x) { float f; memcpy(&f, &x, 4); return f; }
 static inline unsigned __funnelshift_l(unsigned lo, unsigned hi, unsigned s) {
@@ -83,6 +86,47 @@ int main(int argc, char **argv) {
             ok = true;
             const double2 r = cfac_sq(cfac_of(cx(x, y)), ok), w = csq(cx(x, y));
             if (ok && (!same(r.x, w.x) || !same(r.y, w.y))) miss("cfac_sq", x, y);
+        }
+        // products of parts of any size, and with zero parts
+        if (cfac_ok<false>(cx(x, y), cx(u, v))) {
+            bool ok = true;
+            const double2 p = cfac_mul(cfac_of(cx(x, y)), cfac_of(cx(u, v)), ok);
+            const double2 q = cmul(cx(x, y), cx(u, v));
+            if (ok && (!same(p.x, q.x) || !same(p.y, q.y))) miss("cfac_ok", x, u);
+        }
+        if (cfac_ok<true>(cx(x, 0.), cx(u, v))) {
+            bool ok = true;
+            const double2 p = cfac_mul0(cfac_of0(cx(x, 0.)), cfac_of(cx(u, v)), ok);
+            const double2 q = cmul(cx(x, 0.), cx(u, v));
+            if (ok && (!same(p.x, q.x) || !same(p.y, q.y))) miss("cfac_ok0", x, u);
+        }
+        // p 2^ep + q 2^eq on one frame: the rounded sums on p's frame, for q that
+        // stays normal there
+        {
+            const int ep = (int)(g() % 4000) - 2000, d = (int)(g() % 300) - 150;
+            const double2 p = cx(std::ldexp(x, -(int)(g() % 40)), y), q = cx(u, v);
+            if (dfac_ok0(p.x) & dfac_ok0(p.y) & dfac_ok0(u) & dfac_ok0(v)) {
+                bool ok = true;
+                xc r = frame_add(p, ep, q, ep + d, ok);
+                volatile double sx = p.x + std::ldexp(u, d), sy = p.y + std::ldexp(v, d);
+                if (!ok) miss("frame_add range", p.x, u);
+                if (std::ldexp(r.re, r.e - ep) != sx || std::ldexp(r.im, r.e - ep) != sy) miss("frame_add", p.x, u);
+                const xc before = r;
+                ok = true;
+                frame_renorm(r, ok);
+                if (ok && (std::ldexp(r.re, r.e - before.e) != before.re || std::ldexp(r.im, r.e - before.e) != before.im))
+                    miss("frame_renorm", before.re, before.im);
+            }
+        }
+        // |z| < r from upper words
+        {
+            const double h = std::hypot(x, y);
+            const MagF m = mag_of(cx(x, y), 0);
+            if (std::isnan(h)) continue;
+            for (double r : {std::fabs(u), h, std::nextafter(h, INFINITY), h * 1.00001, h * 0.99999, h * 3., h * 0.3, 0.}) {
+                const int lt = mag_lt(m, r);
+                if (lt >= 0 && lt != (h < r ? 1 : 0)) miss("mag_lt", h, r);
+            }
         }
         // thresholds: t itself a square, and |z| drawn near its root too
         const double t = u * u, near = std::sqrt(t) * (1. + ((int)(g() % 5) - 2) * 0x1p-52);
