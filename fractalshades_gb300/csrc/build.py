@@ -34,6 +34,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relax
 SOURCES = {
     "fsg_std.cu": ["-fmad=false"],
     "fsg_perturb.cu": ["-fmad=false"],
+    "fsg_perturb_bs64.cu": ["-fmad=false"],
     "fsg_ref.cu": ["-fmad=false"],
     "fsg_perturb_fe32.cu": [],
     "fsg_perturb_bs32.cu": [],

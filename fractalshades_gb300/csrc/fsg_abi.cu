@@ -346,8 +346,9 @@ int launch_on(fsg_ctx *ctx, const LaunchRes &L, const fsg_calc *calc, const Tile
     W.blocked = perturb && !seg.order && seg.base == 0 && seg.end == tiles_pixels(tiles, ntiles);
     CalcDev C = make_calc(calc);
     // one persistent wave at the kernel's occupancy limit, or the tuned shape
-    // (0: the standard loop's launcher chooses by the size)
-    const int block = calc->block > 0 || !perturb ? calc->block : default_block(calc, perturb);
+    // (0: the launchers of the FP64 kernels choose by the size)
+    const bool fe32 = perturb && calc->mode == FSG_MODE_FE32;
+    const int block = calc->block > 0 || !fe32 ? calc->block : default_block(calc, perturb);
     const int grid = calc->ctas_per_sm > 0 ? -calc->ctas_per_sm : 0;
     if (L.ev0 && seg.first && !seg.keep_time) CK(cudaEventRecord(L.ev0, s), "cudaEventRecord");
     if (!perturb) fsg_launch_std(W, C, grid, block, s);
@@ -871,6 +872,9 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
     if (R.div_iter < R.first_invalid) R.first_invalid = R.div_iter;
     if (R.order < R.first_invalid) R.first_invalid = R.order;
     R.flavor = d->flavor;
+    // (with no side table: its values may be off the axis where the doubles are 0)
+    R.axis = d->flavor != 0 && d->n_xr == 0;
+    for (int i = 0; R.axis && i < len; i++) R.axis = d->Zn[2 * (size_t)i + 1] == 0.;
     R.n_xr = d->n_xr;
     // binomial coefficients C(n, k) as float64, exact for n <= FSG_MN_MAX_EXP
     // (mandelbrot_Mn.py:636-640 math.comb)

@@ -785,6 +785,85 @@ FSG_DEV int bs_frame_tests(const BSFrame &S, float X, float Y, int eX, int eY, f
     return 0;
 }
 
+// One step of flavor 1 in the double form, bs_hess and bs_zn with their products
+// on the integer pipes: false (nothing changed) where one of them is left open.
+// xs = X + xn, ys = Y + yn.  The FP64 pipe sees 24 sums instead of the 69
+// instructions of the plain form: what belongs to the fold's other branch (the
+// reference's own d(XY), with ddiffabsdX = 0) is taken only there.
+// AXIS: the orbit is real (Y = Xb = Ya = 0 at every point: the nuclei that a
+// Newton search from the ship's antenna finds).  A third of the products are then
+// zeros, and a sum with a zero is its other term while that is not 0: they are
+// left out, for 15 sums, and a result that comes out as 0, whose sign they could
+// change, refuses the step.
+template <bool AXIS>
+FSG_DEV bool bs_step_ship(bool hess, double &xn, double &yn, double h[4], double X, double Y, double xs,
+                          double ys, double Xa, double Xb, double Ya, double Yb, double a, double b) {
+    bool ok = true;
+    double x2 = xn;                              // xn + 2 X (X = 0 once per rebase)
+    if (!d_is0(X) | d_is0(xn)) x2 = d_add_here(xn, d_twice(X));
+    const sfac fx = sfac_of(xn), fy = sfac_of(yn), fX = sfac_of(X), fY = sfac_of(Y);
+    // the fold |X Y|: opx its argument's change, `first` its sign at the orbit,
+    // `same` whether the argument keeps it, s1 = ddiffabsdx
+    double opX = 0., opx = sfac_mul(fx, fy, ok);
+    bool first = true, same;
+    if (AXIS) {
+        opx += sfac_mul(fy, fX, ok);
+        ok &= !d_is0(opx) & !d_is0(yn);
+        same = d_ge0(opx);
+    } else {
+        opx = opx + sfac_mul(fx, fY, ok) + sfac_mul(fy, fX, ok);
+        opX = sfac_mul(fX, fY, ok);
+        const double t = opX + opx;
+        first = d_ge0(opX);
+        same = first ? d_ge0(t) : d_le0(t);
+    }
+    const unsigned s1 = first == same ? 0u : 0x80000000u;
+    double fold = opx;
+    if (!AXIS && !same) fold = d_add_here(d_twice(opX), opx);
+    const double y2 = AXIS ? yn : yn + d_twice(Y);
+    const double nx = sfac_mul(fx, sfac_of(x2), ok) - sfac_mul(fy, AXIS ? fy : sfac_of(y2), ok) + a;
+    const double ny = d_twice(d_flip(fold, s1)) - b;
+    if (hess) {
+        const sfac xa = sfac_of(h[0]), xb = sfac_of(h[1]), ya = sfac_of(h[2]), yb = sfac_of(h[3]);
+        const sfac fXa = sfac_of(Xa), fYb = sfac_of(Yb), fs = sfac_of(xs);
+        double da = sfac_mul(xa, fy, ok) + sfac_mul(fx, ya, ok);
+        double db = sfac_mul(xb, fy, ok) + sfac_mul(fx, yb, ok);
+        double nxa = sfac_mul(fs, xa, ok) + sfac_mul(fXa, fx, ok), nxb = sfac_mul(fs, xb, ok);
+        double va, vb;
+        if (AXIS) {
+            da = da + sfac_mul(ya, fX, ok) + sfac_mul(fy, fXa, ok);
+            db = db + sfac_mul(fx, fYb, ok) + sfac_mul(yb, fX, ok);
+            va = sfac_mul(fy, ya, ok);
+            vb = sfac_mul(fy, yb, ok) + sfac_mul(fYb, fy, ok);
+        } else {
+            const sfac fXb = sfac_of(Xb), fYa = sfac_of(Ya), ft = sfac_of(ys);
+            da = da + sfac_mul(xa, fY, ok) + sfac_mul(fx, fYa, ok) + sfac_mul(ya, fX, ok) + sfac_mul(fy, fXa, ok);
+            db = db + sfac_mul(xb, fY, ok) + sfac_mul(fx, fYb, ok) + sfac_mul(yb, fX, ok) + sfac_mul(fy, fXb, ok);
+            nxb += sfac_mul(fXb, fx, ok);
+            va = sfac_mul(ft, ya, ok) + sfac_mul(fYa, fy, ok);
+            vb = sfac_mul(ft, yb, ok) + sfac_mul(fYb, fy, ok);
+        }
+        ok &= !(d_is0(da) | d_is0(db));
+        if (!same) {
+            // ddiffabsdX = 2 s1 times the reference's d(XY)
+            double dXb = d_mul_here(X, Yb);
+            if (!AXIS) {
+                dXb = d_add_here(d_mul_here(Xb, Y), dXb);
+                da = d_add_here(d_twice(d_add_here(d_mul_here(Xa, Y), d_mul_here(X, Ya))), da);
+            }
+            db = d_add_here(d_twice(dXb), db);
+        }
+        nxa = d_twice(nxa) - d_twice(va);
+        nxb = d_twice(nxb) - d_twice(vb);
+        if (AXIS) ok &= !(d_is0(db) | d_is0(nxa) | d_is0(nxb));
+        if (!ok) return false;
+        h[0] = nxa; h[1] = nxb; h[2] = d_twice(d_flip(da, s1)); h[3] = d_twice(d_flip(db, s1));
+    }
+    if (!ok) return false;
+    xn = nx; yn = ny;
+    return true;
+}
+
 template <class T> struct IsDouble { static constexpr bool value = false; };
 template <> struct IsDouble<double> { static constexpr bool value = true; };
 template <class T> struct IsFr { static constexpr bool value = false; };
@@ -820,6 +899,8 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
     T h[4] = {cst<T>(0.f), cst<T>(0.f), cst<T>(0.f), cst<T>(0.f)};
     const fr M2f = fr_from_d(C.M2);
     int w = 0, n = 0; signed char stop = -1; bool dyn = true;
+    // double form: X_w + xn and Y_w + yn of the last test, while they stand
+    double XX_last = 0., YY_last = 0.; bool has_sums = false;
     // calc_orbit snapshots (perturbation.py:1501-1508), the reference's two
     // forms only: the FP32 + exponent instantiation compiles without them
     constexpr bool FR_FORM = IsFr<T>::value;
@@ -938,18 +1019,28 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
                 // the reference compares the double value of |dz| (0 when it
                 // underflows, perturbation.py:1123-1135)
                 const int step = BLAGet<T>::get(R, xn, yn, w, ib);
-                if (step != 0) { apply_bla(step, ib); continue; }
+                if (step != 0) { apply_bla(step, ib); has_sums = false; continue; }
             }
             n += 1;
             nfull++;
             T X, Y;
             BSRef<T>::orbit(R, w, X, Y);
-            if (hess) {
-                T Xa = cst<T>(0.f), Xb = cst<T>(0.f), Ya = cst<T>(0.f), Yb = cst<T>(0.f);
-                if (!dyn) BSRef<T>::hess(R, w, Xa, Xb, Ya, Yb);
-                bs_hess<T>(flavor, h, xn, yn, X, Y, Xa, Xb, Ya, Yb);
+            T Xa = cst<T>(0.f), Xb = cst<T>(0.f), Ya = cst<T>(0.f), Yb = cst<T>(0.f);
+            if (hess && !dyn) BSRef<T>::hess(R, w, Xa, Xb, Ya, Yb);
+            bool taken = false;
+            if constexpr (IsDouble<T>::value && FL == 1) {
+                double xs = XX_last, ys = YY_last;
+                if (!has_sums) {
+                    xs = (d_is0(X) & !d_is0(xn)) ? xn : d_add_here(X, xn);
+                    ys = (d_is0(Y) & !d_is0(yn)) ? yn : d_add_here(Y, yn);
+                }
+                taken = R.axis ? bs_step_ship<true>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b)
+                               : bs_step_ship<false>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b);
             }
-            bs_zn<T>(flavor, xn, yn, X, Y, a, b);
+            if (!taken) {
+                if (hess) bs_hess<T>(flavor, h, xn, yn, X, Y, Xa, Xb, Ya, Yb);
+                bs_zn<T>(flavor, xn, yn, X, Y, a, b);
+            }
             if (n >= C.max_iter) { stop = 0; break; }
             w += 1;
             if (w >= order) w = w % order;
@@ -965,7 +1056,7 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
             const double xs = to_d(xn), ys = to_d(yn);
             const double XXd = xs + Zs.x, YYd = ys + Zs.y;
             if (bs > 0) S.take(n, bs, cx(XXd, YYd));
-            if (d_sq_gt(XXd * XXd + YYd * YYd, C.M2)) { stop = 1; break; }
+            if (fsg_escaped(C, cx(XXd, YYd))) { stop = 1; break; }
             if (w >= div_iter - 1) {
                 xn = from_d<T>(XXd); yn = from_d<T>(YYd);
                 if (hess) {
@@ -995,16 +1086,27 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
         }
         T Xs, Ys;
         BSRef<T>::orbit(R, w, Xs, Ys);
-        T XX = xn + Xs, YY = yn + Ys;
+        T XX, YY;
+        if constexpr (IsDouble<T>::value) {
+            // a sum with 0 is its other term while that is not 0
+            XX = xn; YY = yn;
+            if (!d_is0(Xs) | d_is0(xn)) XX = d_add_here(xn, Xs);
+            if (!d_is0(Ys) | d_is0(yn)) YY = d_add_here(yn, Ys);
+            XX_last = XX; YY_last = YY;
+            has_sums = true;
+        } else {
+            XX = xn + Xs; YY = yn + Ys;
+        }
         if constexpr (ORB_FORM) {
             const double XXd = to_d(XX), YYd = to_d(YY);
             if (bs > 0) S.take(n, bs, cx(XXd, YYd));             // :1641-1651
-            if (d_sq_gt(XXd * XXd + YYd * YYd, C.M2)) { stop = 1; break; }
+            if (fsg_escaped(C, cx(XXd, YYd))) { stop = 1; break; }
         } else {
             if (fr_escaped(XX, YY, M2f, C.M2)) { stop = 1; break; }
         }
         if (w >= div_iter - 1) {
             xn = XX; yn = YY;
+            has_sums = false;
             if (hess) {
                 T Ha, Hb, Hc, Hd;
                 BSRef<T>::hess(R, w, Ha, Hb, Hc, Hd);
@@ -1015,6 +1117,7 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
         dyn = abs_le(XX, xn) && abs_le(YY, yn);
         if (dyn) {
             xn = XX; yn = YY;
+            has_sums = false;
             if (hess) {
                 T Ha, Hb, Hc, Hd;
                 BSRef<T>::hess(R, w, Ha, Hb, Hc, Hd);
@@ -1080,9 +1183,11 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
 }
 
 // the FP32 + exponent kernels hold three 256-thread blocks per SM (at most 85
-// registers a thread)
+// registers a thread), the others two (128): flavor 1 in the double form, 255^2
+// pixels of the period-12 nucleus to 20000 iterations, takes 68 ms with them, 95
+// ms at its own 156 registers and one block, 73 ms at 80 with spills
 template <class T, int FL>
-__global__ void __launch_bounds__(256, IsFr<T>::value ? 3 : 1)
+__global__ void __launch_bounds__(256, IsFr<T>::value ? 3 : 2)
 k_perturb_bs(WorkDev W, CalcDev C) {
     extern __shared__ long long s_start[];          // [W.ntiles + 1], sized at launch
     fsg_load_starts(W, s_start);

@@ -29,6 +29,7 @@ struct RefDev {
     // derivative paths, Xrange form
     const double2 *dZndc_xm; const int *dZndc_xe;
     const double2 *dZndz_xm; const int *dZndz_xe;
+    int axis;                                   // Burning Ship: the whole orbit is real
     // BS Jacobian paths
     const double *dXa, *dXb, *dYa, *dYb;        // [len + 1]
     const double *bs_xpm; const int *bs_xpe;    // Xrange branch: [4][len + 1] dXa, dXb, dYa,
@@ -376,6 +377,16 @@ inline int fsg_auto_grid(K kernel, int grid, int block, long long total, size_t 
     return (int)g;
 }
 
+// Threads per CTA of an FP64 perturbation kernel where the caller leaves it open:
+// 256, or 64 for an image that the SMs hold all at once -- in CTAs of 256 some
+// SMs then hold one more CTA than others and finish that much later.
+template <class K>
+inline int fsg_fp64_block(K kernel, int block, long long total, size_t smem) {
+    if (block > 0) return block;
+    const long long fit = 256LL * fsg_auto_grid(kernel, 0, 256, 1LL << 40, smem);
+    return total <= fit ? 64 : 256;
+}
+
 #ifndef FSG_FIELDLINES_MAX_ITER
 #define FSG_FIELDLINES_MAX_ITER 64
 #endif
@@ -404,6 +415,7 @@ void fsg_launch_normal(const NormalDev &A, cudaStream_t s);
 // at full occupancy
 void fsg_launch_std(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s);
 void fsg_launch_perturb(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s);
+void fsg_launch_perturb_bs(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s);
 void fsg_launch_perturb_bs_fe32(const WorkDev &W, const CalcDev &C, int grid, int block,
                                 cudaStream_t s);
 void fsg_launch_perturb_fe32(const WorkDev &W, const CalcDev &C, int grid, int block,

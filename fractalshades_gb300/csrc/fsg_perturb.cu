@@ -6,8 +6,7 @@
 // models/mandelbrot_Mn.py:626-733 (MN = true, fsg_mn.cuh).  XR = false is the branch with
 // xr_detect_activated False (double deltas), XR = true the Xrange branch
 // (double mantissa + int32 exponent, numba_xr.py semantics).
-// Burning Ship family: perturbation.py:1406-1811 with the closures of
-// models/burning_ship.py:19-60, 535-859 (double deltas).
+// (Burning Ship family: fsg_perturb_bs64.cu.)
 //
 // Built with -fmad=false so that every operation rounds once in the order of
 // the reference source.  One thread iterates one pixel at a time and claims
@@ -521,15 +520,10 @@ __global__ void __launch_bounds__(256) k_perturb_m2(WorkDev W, CalcDev C) {
     fsg_flush_stats(W, itsum, nfull, nbla, nreb);
 }
 
-// Burning Ship family, double deltas: fsg_bs.cuh instantiated on double
-// (compiled here, without FMA contraction)
-template __global__ void k_perturb_bs<double, 0>(WorkDev W, CalcDev C);
-// ... and on float64 Xrange records: the reference's Xrange branch
-template __global__ void k_perturb_bs<xf, 0>(WorkDev W, CalcDev C);
-
 template <bool XR, bool MN, bool ORB>
 static void launch_m2(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s) {
     const size_t sm = fsg_starts_smem(W);
+    block = fsg_fp64_block(k_perturb_m2<XR, MN, ORB>, block, W.total - W.base, sm);
     k_perturb_m2<XR, MN, ORB><<<fsg_auto_grid(k_perturb_m2<XR, MN, ORB>, grid, block,
                                               W.total - W.base, sm), block, sm, s>>>(W, C);
 }
@@ -544,13 +538,7 @@ static void launch_m2_orb(const WorkDev &W, const CalcDev &C, int grid, int bloc
 }
 
 void fsg_launch_perturb(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s) {
-    const size_t sm = fsg_starts_smem(W);
-    if (C.flavor != 0 && C.mode == 1)
-        k_perturb_bs<xf, 0><<<fsg_auto_grid(k_perturb_bs<xf, 0>, grid, block, W.total - W.base, sm),
-                              block, sm, s>>>(W, C);
-    else if (C.flavor != 0)
-        k_perturb_bs<double, 0><<<fsg_auto_grid(k_perturb_bs<double, 0>, grid, block,
-                                                W.total - W.base, sm), block, sm, s>>>(W, C);
+    if (C.flavor != 0) fsg_launch_perturb_bs(W, C, grid, block, s);
     else if (C.backshift > 0)
         launch_m2_orb<true>(W, C, grid, block, s);
     else

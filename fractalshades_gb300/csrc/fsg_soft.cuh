@@ -25,8 +25,32 @@
 
 struct dfac { unsigned s, h, l; };
 
+// a + b and a * b where the code asks for them and nowhere ahead of their branch
+FSG_DEV double d_mul_here(double a, double b) {
+#ifdef __CUDA_ARCH__
+    double r;
+    asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+#else
+    return a * b;
+#endif
+}
+FSG_DEV double d_add_here(double a, double b) {
+#ifdef __CUDA_ARCH__
+    double r;
+    asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    return r;
+#else
+    return a + b;
+#endif
+}
 FSG_DEV unsigned d_hi(double x) { return (unsigned)(dbits(x) >> 32); }
 FSG_DEV unsigned d_lo(double x) { return (unsigned)dbits(x); }
+
+// x with its sign bit xored by s (0 or 0x80000000): the product by 1 or -1
+FSG_DEV double d_flip(double x, unsigned s) {
+    return __hiloint2double((int)(d_hi(x) ^ s), (int)d_lo(x));
+}
 
 // normal, exponent in [-480, 479]: no product of two such leaves the normal range
 #define FSG_FAC_LO (1023u - 480u)
@@ -58,19 +82,29 @@ FSG_DEV double dfac_mul_t(const dfac &a, const dfac &b, bool &ok) {
     const unsigned vh = (unsigned)(v >> 32), vl = (unsigned)v, ul = (unsigned)u;
     const unsigned q = vh >> 21;                       // 1: the product is in [2, 4)
     const unsigned H = vh >> q, L = __funnelshift_r(vl, vh, q), r = __funnelshift_r(ul, vl, q);
-    unsigned up = r >> 31;
+    // the rounding bit, at the top of r; a tie to the even neighbour
+    unsigned top = r;
     if (TIES) {
         const bool below = ((unsigned)t | (ul & q)) != 0u;       // bits under r
-        if (r == 0x80000000u && !below) up = L & 1u;
+        if (r == 0x80000000u && !below) top = L << 31;
     } else {
         ok &= r != 0x80000000u;
     }
     // exponent fields and signs add modulo 2^32 (the exponent of the result is
     // in range); H carries the mantissa's leading bit, which adds 1 to the field
     const unsigned e = a.s + b.s - 0x40000000u + (q << 20);
-    u64 m = ((u64)(H + e) << 32 | L) + up;
-    if (ZERO && vh == 0u) m = (u64)((a.s ^ b.s) & 0x80000000u) << 32;
-    return __longlong_as_double((long long)m);
+    unsigned lo, hi;
+#ifdef __CUDA_ARCH__
+    // (the top bit as the carry of top + top)
+    asm("{ .reg .u32 c; add.cc.u32 c, %2, %2; addc.cc.u32 %0, %3, 0; addc.u32 %1, %4, %5; }"
+        : "=r"(lo), "=r"(hi) : "r"(top), "r"(L), "r"(H), "r"(e));
+#else
+    const u64 m = ((u64)(H + e) << 32 | L) + (top >> 31);
+    lo = (unsigned)m;
+    hi = (unsigned)(m >> 32);
+#endif
+    if (ZERO && vh == 0u) { lo = 0u; hi = (a.s ^ b.s) & 0x80000000u; }
+    return __hiloint2double((int)hi, (int)lo);
 }
 FSG_DEV double dfac_mul(const dfac &a, const dfac &b, bool &ok) {
     return dfac_mul_t<false, false>(a, b, ok);
@@ -137,6 +171,36 @@ FSG_DEV bool cfac_ok(double2 a, double2 b) {
     const unsigned la = min(ax, ay), ha = max(ax, ay), lb = min(bx, by), hb = max(bx, by);
     return (min(la, lb) != 0u) & (max(ha, hb) != 0x7ff00000u) & (la + lb >= 1025u << 20)
            & (ha + hb <= 3068u << 20);
+}
+
+// ---------------------------------------------------------------------------
+// A factor of any size, for loops whose values range from 1 to far below
+// 2^-480: its exponent field f tells products that are normal from those that
+// round to zero (a zero factor, or a product below 2^-1075) and from the rest
+// (subnormal results, overflow, infinities and NaN), which clear ok.
+// ---------------------------------------------------------------------------
+struct sfac { unsigned s, h, l; int f; };
+#define FSG_F_ZERO (-10000)
+#define FSG_F_SUB 5000
+#define FSG_F_INF 20000
+FSG_DEV sfac sfac_of(double x, int k = 0) {
+    const dfac d = dfac_of(x, k);
+    const int e = (int)(d_hi(x) >> 20 & 0x7ffu);
+    sfac f;
+    f.s = d.s; f.h = d.h; f.l = d.l;
+    f.f = e == 0x7ff ? FSG_F_INF : e == 0 ? (d_is0(x) ? FSG_F_ZERO : FSG_F_SUB) : e + k;
+    return f;
+}
+FSG_DEV double sfac_mul(const sfac &a, const sfac &b, bool &ok) {
+    dfac p, q;
+    p.s = a.s; p.h = a.h; p.l = a.l;
+    q.s = b.s; q.h = b.h; q.l = b.l;
+    bool kept = true;
+    const double m = dfac_mul(p, q, kept);
+    const int e = a.f + b.f;
+    const bool zero = e <= 968;                 // below 2^(968 - 2044) = 2^-1076
+    ok &= zero | (kept & (unsigned)(e - 1025) <= 3068u - 1025u);
+    return zero ? d_zero(((a.s ^ b.s) >> 31) != 0u) : m;
 }
 
 // cmul, by the integer products where they can be (out of line elsewhere)

@@ -46,10 +46,6 @@ __device__ __forceinline__ void std_opt_take(StdOpt<OPT> &o, const CalcDev &C, i
     if constexpr (OPT) { if (C.backshift > 0) o.S.take(n, C.backshift, z); }
 }
 
-// x with its sign bit xored by s (0 or 0x80000000): the product by 1 or -1
-__device__ __forceinline__ double d_flip(double x, unsigned s) {
-    return __hiloint2double(__double2hiint(x) ^ (int)s, __double2loint(x));
-}
 struct CoopLane { unsigned k, neg; bool add; double g; };
 
 // Power-2 and power-n Mandelbrot: the complex state
