@@ -27,93 +27,173 @@ __device__ __forceinline__ xc orbit_xr(const RefDev &R, int i) {
     return xr_from(z);
 }
 
-// The orbit fields the sequential loops read, held in registers: the loops
-// store into the paths, which the compiler cannot prove apart from the
-// descriptor, so reading them through it would reload them every step
-struct OrbitView {
-    const double2 *__restrict__ Zn;
-    const int *__restrict__ xr_slot;
-    const double2 *__restrict__ xr_m;
-    const int *__restrict__ xr_e;
-    int n_xr, nexp;
-    __device__ __forceinline__ explicit OrbitView(const RefDev &R)
-        : Zn(R.Zn), xr_slot(R.xr_slot), xr_m(R.xr_m), xr_e(R.xr_e), n_xr(R.n_xr), nexp(R.nexp) {}
-    __device__ __forceinline__ xc xr(int i) const {
-        int slot = n_xr ? xr_slot[i] : -1;
-        if (slot >= 0) return xc_make(xr_m[slot].x, xr_m[slot].y, xr_e[slot]);
-        return xr_from(Zn[i]);
-    }
+// Sequential form (orbits up to FSG_PATH_SCAN_MIN = 8192 points), in the
+// reference's order: D_i = a_i D_{i-1} (+ s), a_i = df/dz(Z_{i-1}).  The chain of
+// one step after the other is all of the time: an FP64 instruction returns after
+// 63 clocks, its result reaches an integer test after 40 more, a vote or a
+// shuffle takes 30 and a taken branch 20.  Two lanes walk the chain, one for
+// each part of D: two products, their sum, the sum with s, and the parts change
+// hands.  The Xrange tests are read every FSG_PATH_RUN steps; steps that ask for
+// more than the chain does are taken again.  The block's threads turn
+// FSG_PATH_PART orbit points at a time into a_i in shared memory, and write the
+// part's results.  2474 points, Xrange: 1.80 ms with one thread doing everything,
+// 0.55 ms like this.  The paths are zero-filled by the host (cudaMemsetAsync)
+// before the launch.
+#define FSG_PATH_PART 256
+#define FSG_PATH_THREADS 128
+#define FSG_PATH_RUN 8          // steps between two looks at the Xrange tests
+struct PathShared {
+    double2 a[FSG_PATH_PART], out[FSG_PATH_PART];
+    int ae[FSG_PATH_PART], oe[FSG_PATH_PART];
 };
 
-// Sequential form (orbits up to FSG_PATH_SCAN_MIN = 8192 points): one thread, the
-// reference's order, the previous value carried in registers.  The paths are
-// zero-filled by the host (cudaMemsetAsync) before the launch.
-__global__ void k_dzndc_m2(const RefDev *Rp, double2 *__restrict__ out_std,
-                           double2 *__restrict__ out_xm, int *__restrict__ out_xe,
-                           int xr_mode, double scale_m, int scale_e) {
-    const RefDev &R = *Rp;
-    const OrbitView O(R);
-    const int len = R.len, order = R.order, nexp = O.nexp;
-    const int valid = len < R.div_iter ? len : R.div_iter;
-    int i;
-    if (xr_mode) {
-        const xc sc = xc_make(scale_m, 0., scale_e);
-        xc prev = xc_zero();
-        for (i = 1; i < valid; i++) {
-            xc v = xr_add(xr_mul(mn_dfdz_x(nexp, O.xr(i - 1)), prev), sc);
-            out_xm[i] = cx(v.re, v.im); out_xe[i] = v.e;
-            prev = v;
+// xr_add(xr_mul(a 2^ae, D), s 2^se), or caddr(cmul(a, D), s)
+template <bool XR>
+static __device__ __noinline__ xc path_step_full(double2 a, int ae, xc D, double s, int se, bool affine) {
+    if (!XR) {
+        const double2 m = cmul(a, xm(D)), r = affine ? caddr(m, s) : m;
+        return xc_make(r.x, r.y, 0);
+    }
+    const xc r = xr_mul(xc_make(a.x, a.y, ae), D);
+    return affine ? xr_add(r, xc_make(s, 0., se)) : r;
+}
+
+// indices [first, valid) from prev at first - 1; returns the last value (warp 0)
+template <bool XR, bool AFFINE>
+__device__ __forceinline__ xc path_seq(const RefDev &R, PathShared &S, int first, int valid, xc prev,
+                                       double s, int se, double2 *__restrict__ out_std,
+                                       double2 *__restrict__ out_xm, int *__restrict__ out_xe) {
+    const int role = threadIdx.x & 1;                // 0: real part, 1: imaginary
+    const unsigned minus = role ? 0u : 0x80000000u;
+    const bool s0 = AFFINE && d_is0(s);
+    double own = role ? prev.im : prev.re, oth = role ? prev.re : prev.im;
+    int e = prev.e;
+    for (int base = first; base < valid; base += FSG_PATH_PART) {
+        const int cnt = min(FSG_PATH_PART, valid - base);
+        for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
+            xc a;
+            if (XR) {
+                a = mn_dfdz_x(R.nexp, orbit_xr(R, base + k - 1));
+            } else {
+                const double2 d = mn_dfdz(R.nexp, R.Zn[base + k - 1]);
+                a = xc_make(d.x, d.y, 0);
+            }
+            S.a[k] = xm(a); S.ae[k] = a.e;
         }
-        i -= 1;
-        if (i == order - 1) {
-            xc v = xr_add(xr_mul_s(mn_dfdz(nexp, O.Zn[i]), prev), sc);
-            out_xm[0] = cx(v.re, v.im); out_xe[0] = v.e;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            for (int k0 = 0; k0 < cnt; k0 += FSG_PATH_RUN) {
+                const int k1 = min(k0 + FSG_PATH_RUN, cnt);
+                const double own0 = own, oth0 = oth;
+                const int e0 = e;
+                bool odd = k1 - k0 < FSG_PATH_RUN;
+                double2 as[FSG_PATH_RUN];
+                int es[FSG_PATH_RUN];
+                if (!odd) {
+#pragma unroll
+                    for (int j = 0; j < FSG_PATH_RUN; j++) { as[j] = S.a[k0 + j]; es[j] = S.ae[k0 + j]; }
+                }
+#pragma unroll
+                for (int j = 0; j < FSG_PATH_RUN; j++) {
+                    if (odd && j == 0) break;
+                    const int k = k0 + j;
+                    const double2 a = as[j];
+                    if (XR) {
+                        // xr_add takes D's product and s on the larger of their
+                        // exponents; the product's share of that shift goes to a,
+                        // ahead of the chain (a power of two: the same bits while
+                        // nothing leaves the normal range)
+                        const int e1 = (int)((unsigned)e + (unsigned)es[j]);
+                        const int t = AFFINE ? min(e1 - se, 0) : 0;
+                        const double u = role || !AFFINE ? 0. : xr_exp2_shift(s, min(se - e1, 0));
+                        const double m = xr_exp2_shift(a.x, t) * own
+                                         + xr_exp2_shift(d_flip(a.y, minus), t) * oth;
+                        own = AFFINE ? m + u : m;
+                        e = AFFINE ? max(e1, se) : e1;
+                        // xr_mul's lazy renormalisation (of the product before the
+                        // shift; a zero part asks for it too), and what the shift
+                        // does not cover
+                        odd |= ((unsigned)(d_field(m) - t - 923) > 200u) | (t < -800) | s0
+                               | (d_field_min(a) == 0);
+                        if (threadIdx.x == 0) S.oe[k] = e;
+                    } else {
+                        // cmul(a, D): a.x D.x - a.y D.y, a.x D.y + a.y D.x
+                        const double m = a.x * own + d_flip(a.y, minus) * oth;
+                        own = AFFINE ? m + (role ? 0. : s) : m;
+                    }
+                    oth = __shfl_xor_sync(0xffffffffu, own, 1);
+                    if (threadIdx.x < 2) ((double *)&S.out[k])[role] = own;
+                }
+                if (__any_sync(0xffffffffu, odd)) {
+                    // these steps again (and what is left of the part), with the
+                    // reference's operations
+                    xc r = role ? xc_make(oth0, own0, e0) : xc_make(own0, oth0, e0);
+                    for (int k = k0; k < k1; k++) {
+                        r = path_step_full<XR>(S.a[k], S.ae[k], r, s, se, AFFINE);
+                        if (threadIdx.x == 0) { S.out[k] = xm(r); S.oe[k] = r.e; }
+                    }
+                    own = role ? r.im : r.re;
+                    oth = role ? r.re : r.im;
+                    e = r.e;
+                }
+            }
         }
+        __syncthreads();
+        for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
+            if (XR) { out_xm[base + k] = S.out[k]; out_xe[base + k] = S.oe[k]; }
+            else out_std[base + k] = S.out[k];
+        }
+        // (the next part's values overwrite these)
+        __syncthreads();
+    }
+    return xc_make(role ? oth : own, role ? own : oth, e);
+}
+
+template <bool XR>
+__device__ __forceinline__ void dzndc_seq(const RefDev &R, PathShared &S, double2 *out_std, double2 *out_xm,
+                                          int *out_xe, double scale_m, int scale_e) {
+    const int valid = R.len < R.div_iter ? R.len : R.div_iter;
+    const double s = XR ? scale_m : ldexp_d(scale_m, scale_e);
+    const xc prev = path_seq<XR, true>(R, S, 1, valid, xc_zero(), s, scale_e, out_std, out_xm, out_xe);
+    const int i = valid > 1 ? valid - 1 : 0;
+    if (threadIdx.x != 0 || i != R.order - 1) return;
+    if (XR) {
+        const xc v = xr_add(xr_mul_s(mn_dfdz(R.nexp, R.Zn[i]), prev), xc_make(scale_m, 0., scale_e));
+        out_xm[0] = xm(v); out_xe[0] = v.e;
     } else {
-        const double scale = ldexp_d(scale_m, scale_e);
-        double2 prev = cx(0., 0.);
-        double2 znext = O.Zn[0];
-        for (i = 1; i < valid; i++) {
-            const double2 z = znext;
-            znext = O.Zn[i];
-            prev = caddr(cmul(mn_dfdz(nexp, z), prev), scale);
-            out_std[i] = prev;
-        }
-        i -= 1;
-        if (i == order - 1) out_std[0] = caddr(cmul(mn_dfdz(nexp, O.Zn[i]), prev), scale);
+        out_std[0] = caddr(cmul(mn_dfdz(R.nexp, R.Zn[i]), xm(prev)), s);
+    }
+}
+template <bool XR>
+__device__ __forceinline__ void dzndz_seq(const RefDev &R, PathShared &S, double2 *out_std, double2 *out_xm,
+                                          int *out_xe) {
+    const int len = R.len, valid = len < R.div_iter ? len : R.div_iter;
+    const xc prev = path_seq<XR, false>(R, S, 2, valid, xc_make(1., 0., 0), 0., 0, out_std, out_xm, out_xe);
+    if (threadIdx.x != 0) return;
+    const int i = valid > 2 ? valid - 1 : 1;         // prev holds the path at i
+    if (XR) {
+        out_xm[1] = cx(1., 0.); out_xe[1] = 0;
+        const xc v = xr_mul(mn_dfdz_x(R.nexp, orbit_xr(R, i)), prev);
+        out_xm[len] = xm(v); out_xe[len] = v.e;
+    } else {
+        out_std[1] = cx(1., 0.);
+        out_std[len] = cmul(mn_dfdz(R.nexp, R.Zn[i]), xm(prev));
     }
 }
 
-__global__ void k_dzndz_m2(const RefDev *Rp, double2 *__restrict__ out_std,
-                           double2 *__restrict__ out_xm, int *__restrict__ out_xe, int xr_mode) {
+// block 0: dZndc, block 1: dZndz (whichever are asked for)
+__global__ void __launch_bounds__(FSG_PATH_THREADS)
+k_paths_m2(const RefDev *Rp, double2 *c_std, double2 *c_xm, int *c_xe, double2 *z_std, double2 *z_xm,
+           int *z_xe, int xr_mode, int want_c, int want_z, double scale_m, int scale_e) {
+    __shared__ PathShared S;
     const RefDev &R = *Rp;
-    const OrbitView O(R);
-    const int len = R.len, nexp = O.nexp;
-    const int valid = len < R.div_iter ? len : R.div_iter;
-    int i;
-    if (xr_mode) {
-        out_xm[1] = cx(1., 0.); out_xe[1] = 0;
-        xc prev = xc_make(1., 0., 0);
-        for (i = 2; i < valid; i++) {
-            xc v = xr_mul(mn_dfdz_x(nexp, O.xr(i - 1)), prev);
-            out_xm[i] = cx(v.re, v.im); out_xe[i] = v.e;
-            prev = v;
-        }
-        i -= 1;          // >= 1: prev holds the path at i
-        xc v = xr_mul(mn_dfdz_x(nexp, O.xr(i)), prev);
-        out_xm[len] = cx(v.re, v.im); out_xe[len] = v.e;
-    } else {
-        out_std[1] = cx(1., 0.);
-        double2 prev = cx(1., 0.);
-        double2 znext = O.Zn[1];
-        for (i = 2; i < valid; i++) {
-            const double2 z = znext;
-            znext = O.Zn[i];
-            prev = cmul(mn_dfdz(nexp, z), prev);
-            out_std[i] = prev;
-        }
-        i -= 1;          // >= 1: prev holds the path at i
-        out_std[len] = cmul(mn_dfdz(nexp, O.Zn[i]), prev);
+    const bool c = want_c && blockIdx.x == 0;
+    if (c) {
+        if (xr_mode) dzndc_seq<true>(R, S, c_std, c_xm, c_xe, scale_m, scale_e);
+        else dzndc_seq<false>(R, S, c_std, c_xm, c_xe, scale_m, scale_e);
+    } else if (want_z) {
+        if (xr_mode) dzndz_seq<true>(R, S, z_std, z_xm, z_xe);
+        else dzndz_seq<false>(R, S, z_std, z_xm, z_xe);
     }
 }
 
@@ -838,9 +918,7 @@ void fsg_build_paths_m2(const RefDev *Rd, int len, double2 *dzndc, double2 *dznd
         } else {
             cudaMemsetAsync(dzndc, 0, 16 * (size_t)(len + 1), s);
         }
-        if (!scan) {
-            k_dzndc_m2<<<1, 1, 0, s>>>(Rd, dzndc, dzndc_xm, dzndc_xe, xr_mode, scale_m, scale_e);
-        } else {
+        if (scan) {
             build_path_scan(Rd, len, 1, valid, xr_mode, 1, scale_m, scale_e, xc_host(0., 0., 0), dzndc,
                             dzndc_xm, dzndc_xe, s);
             k_dzndc_tail<<<1, 1, 0, s>>>(Rd, dzndc, dzndc_xm, dzndc_xe, xr_mode, scale_m, scale_e);
@@ -853,14 +931,16 @@ void fsg_build_paths_m2(const RefDev *Rd, int len, double2 *dzndc, double2 *dznd
         } else {
             cudaMemsetAsync(dzndz, 0, 16 * (size_t)(len + 2), s);
         }
-        if (!scan) {
-            k_dzndz_m2<<<1, 1, 0, s>>>(Rd, dzndz, dzndz_xm, dzndz_xe, xr_mode);
-        } else {
+        if (scan) {
             build_path_scan(Rd, len, 2, valid, xr_mode, 0, 0., 0, xc_host(1., 0., 0), dzndz,
                             dzndz_xm, dzndz_xe, s);
             k_dzndz_tail<<<1, 1, 0, s>>>(Rd, dzndz, dzndz_xm, dzndz_xe, xr_mode);
         }
     }
+    if (!scan && (want_dzndc || want_dzndz))
+        k_paths_m2<<<(want_dzndc ? 1 : 0) + (want_dzndz ? 1 : 0), FSG_PATH_THREADS, 0, s>>>(
+            Rd, dzndc, dzndc_xm, dzndc_xe, dzndz, dzndz_xm, dzndz_xe, xr_mode, want_dzndc, want_dzndz,
+            scale_m, scale_e);
 }
 void fsg_build_paths_bs_xr(const RefDev *Rd, int len, double *pm, int *pe, double scale_m,
                            int scale_e, cudaStream_t s) {
