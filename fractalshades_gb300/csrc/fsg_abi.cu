@@ -248,6 +248,7 @@ CalcDev make_calc(const fsg_calc *c) {
     d.logd = log(c->nexp ? (double)c->nexp : 2.);
     d.backshift = c->backshift;
     d.d2 = c->calc_d2zndc2;
+    d.axis = 0;
     fsg_calc_thresholds(d);
     return d;
 }
@@ -268,6 +269,7 @@ TileDev make_tile(const fsg_tile &t) {
     d.pot = t.potential; d.dem = t.dem;
     d.dzs = t.dzndc_scale_e;
     d.i_orb = t.i_znorbit;
+    d.axis = t.ref ? t.ref->host.axis : 0;
     d.proj = t.proj; d.ph = t.proj_h; d.pht_re = t.proj_ht_re; d.pht_im = t.proj_ht_im;
     return d;
 }
@@ -345,6 +347,8 @@ int launch_on(fsg_ctx *ctx, const LaunchRes &L, const fsg_calc *calc, const Tile
     // (a segment of a streamed call must run the pixels of its own range)
     W.blocked = perturb && !seg.order && seg.base == 0 && seg.end == tiles_pixels(tiles, ntiles);
     CalcDev C = make_calc(calc);
+    C.axis = 1;
+    for (int i = 0; i < ntiles; i++) C.axis &= tiles[i].axis;
     // one persistent wave at the kernel's occupancy limit, or the tuned shape
     // (0: the launchers of the FP64 kernels choose by the size)
     const bool fe32 = perturb && calc->mode == FSG_MODE_FE32;

@@ -758,6 +758,80 @@ FSG_DEV void bs_frame_step_zero(int flavor, bool hess, BSFrame &S, float4 Hm, in
     frame_set_scale(S);
 }
 
+// bs_frame_step for flavor 1 where the orbit is real (Y = 0 and Hm.y = Hm.z = 0 at
+// every point): the fold's argument is 0 at the orbit, so its branch is the sign
+// of the change, and the terms with zeros are left out.  The roundings are those
+// of the general form's contracted sums with those terms 0 (spelled out where a
+// shorter sum would contract otherwise).
+template <bool DEEP>
+FSG_DEV void bs_frame_step_axis1(bool hess, BSFrame &S, float X, float Y, float4 Hm, int g,
+                                 bool zero_ref) {
+    const float s = DEEP ? 0.f : S.s, ux = S.ux, uy = S.uy;
+    const float xs = DEEP ? 0.f : ux * s, ys = DEEP ? 0.f : uy * s;
+    const float xx2 = ux * (DEEP ? 2.f * X : xs + 2.f * X);
+    const float yy2 = uy * (DEEP ? 2.f * Y : ys + 2.f * Y);
+    const float o1 = DEEP ? __fmul_rn(uy, X) : fmaf(uy, X, __fmul_rn(ux, ys));
+    const bool neg = o1 < 0.f;
+    const float v1 = neg ? -o1 : o1, dx1 = neg ? -1.f : 1.f;
+    if (hess) {
+        const bool hz = zero_ref || (Hm.x == 0.f && Hm.w == 0.f);
+        float k1 = 0.f, dXb = 0.f;
+        if (!hz) {
+            const bool need0 = neg && X != 0.f;
+            if (g + S.E - S.F > 60) frame_raise_F(S, g + S.E - 30);
+            if (need0) {
+                if (g - S.F > 60) frame_raise_F(S, g - 30);
+                dXb = __fmul_rn(__fmul_rn(X, Hm.w), fr_p2c(g - S.F));
+            }
+            k1 = fr_p2c(g + S.E - S.F);
+        } else {
+            Hm = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const float h0 = S.h[0], h1 = S.h[1], h2 = S.h[2], h3 = S.h[3];
+        float nxa, nxb, dxa, dxb;
+        if (DEEP) {
+            nxa = 2.f * (X * h0 + Hm.x * ux * k1) - 2.f * (Y * h2);
+            nxb = 2.f * (X * h1) - 2.f * (Y * h3 + Hm.w * uy * k1);
+            dxa = fmaf(__fmul_rn(uy, Hm.x), k1, __fmul_rn(h2, X));
+            dxb = fmaf(__fmul_rn(ux, Hm.w), k1, __fmul_rn(h3, X));
+        } else {
+            nxa = 2.f * ((X + xs) * h0 + Hm.x * ux * k1) - 2.f * __fmul_rn(Y + ys, h2);
+            nxb = 2.f * __fmul_rn(X + xs, h1) - 2.f * ((Y + ys) * h3 + Hm.w * uy * k1);
+            dxa = fmaf(__fmul_rn(uy, Hm.x), k1, fmaf(h2, X, __fmul_rn(h0 * uy + ux * h2, s)));
+            dxb = fmaf(__fmul_rn(ux, Hm.w), k1, fmaf(h3, X, __fmul_rn(h1 * uy + ux * h3, s)));
+        }
+        S.h[0] = nxa; S.h[1] = nxb;
+        S.h[2] = 2.f * (dx1 * dxa);
+        S.h[3] = neg ? 2.f * fmaf(-2.f, dXb, -dxb) : 2.f * dxb;
+    }
+    S.ux = xx2 - yy2 + S.cux;
+    S.uy = 2.f * v1 - S.cuy;
+}
+
+// bs_frame_step_zero for flavor 1 right after a rebase (the reference Hessian
+// reads as 0): products of deltas and c alone.
+FSG_DEV void bs_frame_zero1(bool hess, BSFrame &S) {
+    const int E = S.E;
+    const int En = max(2 * E, frame_ec(S) - 100);
+    const float s = fr_p2c(2 * E - En), ux = S.ux, uy = S.uy;
+    const float xs = ux * s, ys = uy * s;
+    const float xy = __fmul_rn(ux, ys);
+    const bool neg = xy < 0.f;
+    if (hess) {
+        const float h0 = S.h[0], h1 = S.h[1], h2 = S.h[2], h3 = S.h[3];
+        const float dxa = __fmul_rn(h0 * uy + ux * h2, s), dxb = __fmul_rn(h1 * uy + ux * h3, s);
+        S.h[0] = 2.f * __fmul_rn(xs, h0) - 2.f * __fmul_rn(ys, h2);
+        S.h[1] = 2.f * __fmul_rn(xs, h1) - 2.f * __fmul_rn(ys, h3);
+        S.h[2] = neg ? -2.f * dxa : 2.f * dxa;
+        S.h[3] = neg ? -2.f * dxb : 2.f * dxb;
+    }
+    if (S.F != FR_ZERO_E) S.F += En - E;
+    S.E = En;
+    frame_set_scale(S);
+    S.ux = ux * xs - uy * ys + S.cux;
+    S.uy = 2.f * (neg ? -xy : xy) - S.cuy;
+}
+
 // |X + d| <= |d| for one component (d = du 2^E), as the fr values round:
 // true when X = 0 or |X| < 2^-25 |d| (X + d rounds to d), false when
 // |d| < |X| / 2; open otherwise
@@ -871,11 +945,13 @@ template <> struct IsFr<fr> { static constexpr bool value = true; };
 template <class T> struct IsXr { static constexpr bool value = false; };
 template <> struct IsXr<xf> { static constexpr bool value = true; };
 
-// FL: the flavor as a compile-time constant (1..5), or 0 to read C.flavor
-template <class T, int FL>
+// FL: the flavor as a compile-time constant (1..5), or 0 to read C.flavor.  AXIS:
+// every reference of the launch is real (RefDev.axis), flavor 1
+template <class T, int FL, bool AXIS>
 FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
-                      unsigned long long &nfull, unsigned long long &nbla,
-                      unsigned long long &nreb, unsigned long long &itsum) {
+                      unsigned long long &full_, unsigned long long &bla_,
+                      unsigned long long &reb_, unsigned long long &itsum) {
+    unsigned nfull = 0, nbla = 0, nreb = 0;
     const TileDev &Tl = T_;
     const RefDev &R = *Tl.ref;
     const long long np = (long long)Tl.nx * Tl.ny;
@@ -960,7 +1036,12 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
                     float4 Hm = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (hess && !dyn) Hm = __ldg(&R.bs_fh[w]);
                     if (fz.x & 4) {
-                        bs_frame_step_zero(flavor, hess, Fm, Hm, fz.y, dyn);
+                        if (FL == 1 && dyn) bs_frame_zero1(hess, Fm);
+                        else bs_frame_step_zero(flavor, hess, Fm, Hm, fz.y, dyn);
+                    } else if (AXIS) {
+                        const float4 fa = __ldg(&R.bs_fa[w]);
+                        if (Fm.s == 0.f) bs_frame_step_axis1<true>(hess, Fm, fa.x, fa.y, Hm, fz.y, dyn);
+                        else bs_frame_step_axis1<false>(hess, Fm, fa.x, fa.y, Hm, fz.y, dyn);
                     } else {
                         const float4 fa = __ldg(&R.bs_fa[w]);
                         const int eX = __float_as_int(fa.z), eY = __float_as_int(fa.w);
@@ -989,7 +1070,7 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
                     if (fz.x & 2) {
                         const float4 fb = __ldg(&R.bs_fa[w]);
                         res = bs_frame_tests(Fm, fb.x, fb.y, __float_as_int(fb.z),
-                                             __float_as_int(fb.w), M2s, divr);
+                                             AXIS ? FR_ZERO_E : __float_as_int(fb.w), M2s, divr);
                     }
                     if (res == 0) { dyn = false; continue; }
                     if (res == 1) { stop = 1; frame_out(Fm, xn, yn, h); return 0; }
@@ -1034,8 +1115,7 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
                     xs = (d_is0(X) & !d_is0(xn)) ? xn : d_add_here(X, xn);
                     ys = (d_is0(Y) & !d_is0(yn)) ? yn : d_add_here(Y, yn);
                 }
-                taken = R.axis ? bs_step_ship<true>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b)
-                               : bs_step_ship<false>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b);
+                taken = bs_step_ship<AXIS>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b);
             }
             if (!taken) {
                 if (hess) bs_hess<T>(flavor, h, xn, yn, X, Y, Xa, Xb, Ya, Yb);
@@ -1180,13 +1260,14 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
     double absd = 0.5 * (hypot(hd[0] + hd[3], hd[1] - hd[2]) + hypot(hd[0] - hd[3], hd[1] + hd[2]));
     fsg_epilogue(Tl, C, ip, cx(xo, yo), absd, n);
     itsum += (unsigned long long)n;
+    full_ += nfull; bla_ += nbla; reb_ += nreb;
 }
 
 // the FP32 + exponent kernels hold three 256-thread blocks per SM (at most 85
 // registers a thread), the others two (128): flavor 1 in the double form, 255^2
 // pixels of the period-12 nucleus to 20000 iterations, takes 68 ms with them, 95
 // ms at its own 156 registers and one block, 73 ms at 80 with spills
-template <class T, int FL>
+template <class T, int FL, bool AXIS>
 __global__ void __launch_bounds__(256, IsFr<T>::value ? 3 : 2)
 k_perturb_bs(WorkDev W, CalcDev C) {
     extern __shared__ long long s_start[];          // [W.ntiles + 1], sized at launch
@@ -1196,7 +1277,7 @@ k_perturb_bs(WorkDev W, CalcDev C) {
     while (true) {
         if (!fsg_claim_poll(W, s_start, t, ip)) break;
         const unsigned long long before = itsum;
-        pixel_bs<T, FL>(W.tiles[t], C, ip, nfull, nbla, nreb, itsum);
+        pixel_bs<T, FL, AXIS>(W.tiles[t], C, ip, nfull, nbla, nreb, itsum);
         fsg_account(W, itsum - before);
     }
     fsg_flush_stats(W, itsum, nfull, nbla, nreb);

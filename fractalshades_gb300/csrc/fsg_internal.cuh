@@ -91,6 +91,7 @@ struct TileDev {
     int dzs;                                   // dzndc scale 2^dzs over the reference's
     int i_orb;                                 // Z row of the orbit point
     int proj;                                  // 0 Cartesian, 1 Expmap
+    int axis;                                  // the reference's RefDev.axis
     double ph, pht_re, pht_im;                 // Expmap: exp(ph + pht * pix)
 };
 
@@ -132,6 +133,7 @@ struct CalcDev {
     double logd;                               // log of the degree (potential)
     int backshift;                             // > 0: orbit point n - backshift
     int d2;                                    // standard loop: d2zndc2 in row 3
+    int axis;                                  // Burning Ship: every tile's reference is real
     SqBound esc, stat;                         // M2, eps2 on exponents (fsg_soft.cuh)
 };
 

@@ -155,7 +155,7 @@ extern "C" int fsg_std_tiles_noalloc(const fsg_calc *calc, const fsg_tile *tiles
     C.mode = FSG_MODE_FP64; C.calc_dzndc = 1; C.interior = 0; C.bla = 0;
     C.flavor = calc->flavor; C.xrsem = 0;
     C.nexp = calc->nexp; C.logd = log(calc->nexp ? (double)calc->nexp : 2.);
-    C.backshift = 0; C.d2 = 0;
+    C.backshift = 0; C.d2 = 0; C.axis = 0;
     fsg_calc_thresholds(C);
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
