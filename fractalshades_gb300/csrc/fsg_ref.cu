@@ -571,62 +571,64 @@ __device__ __forceinline__ void runs_norm(double2 &m, int &e) {
 __device__ __forceinline__ int4 runs_pack2(double2 m, int e, int e2) {
     return make_int4(__float_as_int((float)m.x), __float_as_int((float)m.y), e, e2);
 }
+//
+// Bound by the FP64 latency of the eight dependent steps (a few thousand
+// entries leave most SMs idle), so two lanes share an entry: the even one takes
+// P, a and R, the odd one Q, b and S -- the same chain with another start --
+// and they exchange the parts of the packed words at the end.  2474 entries:
+// 47 us with one thread an entry, 26 us with two.
 __global__ void k_fe_runs(const RefDev *Rp, const int4 *Zp, const int4 *Df, int len, int4 *out) {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, w = t >> 1;
+    const bool odd = t & 1;
+    // the lanes of an entry agree on every branch; a warp's last entries may
+    // lie past the end
+    const unsigned am = __ballot_sync(0xffffffffu, w <= len);
     if (w > len) return;
     int4 *o = out + 5 * (size_t)w;
     const int k = 8 - (w & 7);
     bool ok = k >= 2 && w + k <= len;
-    double2 P = cx(1., 0.), Q = cx(0., 0.), Rm = cx(0., 0.), Sm = cx(0., 0.);
-    int eR = 0, eS = 0;
-    double amax = 0., bmax = 0., z2max = 0.;
+    double2 P = cx(odd ? 0. : 1., 0.), Rm = cx(0., 0.);      // (Q and S in the odd lane)
+    int eR = 0;
+    double amax = 0., z2max = 0.;
     for (int j = 0; j < k && ok; j++) {
         const int4 z = Zp[w + j];
         if (z.z == FE_ZERO_E) { ok = false; break; }
         const double sc = ldexp(1., -z.z);
         amax = fmax(amax, hypot(P.x, P.y) * sc);
-        bmax = fmax(bmax, hypot(Q.x, Q.y) * sc);
         const double2 T = cx((double)__int_as_float(z.x), (double)__int_as_float(z.y));
-        if (j >= 1) z2max = fmax(z2max, T.x * T.x + T.y * T.y);
+        if (!odd && j >= 1) z2max = fmax(z2max, T.x * T.x + T.y * T.y);
         if (Df) {
             const int4 d = Df[w + j];
+            Rm = cmul(T, Rm);
             if (d.z != FE_ZERO_E) {
                 const double2 D2 = cx(2. * (double)__int_as_float(d.x), 2. * (double)__int_as_float(d.y));
-                Rm = cmul(T, Rm);
-                Sm = cmul(T, Sm);
                 runs_acc(Rm, eR, cmul(D2, P), d.z);
-                runs_acc(Sm, eS, cmul(D2, Q), d.z);
-            } else {
-                Rm = cmul(T, Rm);
-                Sm = cmul(T, Sm);
             }
             runs_norm(Rm, eR);
             if (eR == FE_ZERO_E) eR = 0;
-            runs_norm(Sm, eS);
-            if (eS == FE_ZERO_E) eS = 0;
         }
         P = cmul(T, P);
-        Q = cadd(cmul(T, Q), cx(1., 0.));
+        if (odd) P = cadd(P, cx(1., 0.));
     }
-    if (!ok) {
-        o[4] = make_int4(0, 0, 0, 0);
-        return;
-    }
-    int eP = 0, eQ = 0;
+    int eP = 0, ea = 0;
     runs_norm(P, eP);
-    runs_norm(Q, eQ);
-    const bool r0 = Rm.x == 0. && Rm.y == 0., s0 = Sm.x == 0. && Sm.y == 0.;
-    o[0] = runs_pack2(P, eP, eQ);
-    o[1] = make_int4(__float_as_int((float)Q.x), __float_as_int((float)Q.y),
-                     __float_as_int((float)Rm.x), __float_as_int((float)Rm.y));
-    o[2] = make_int4(r0 ? FE_ZERO_E : eR, s0 ? FE_ZERO_E : eS,
-                     __float_as_int((float)Sm.x), __float_as_int((float)Sm.y));
-    int ea = 0, eb = 0;
-    const double ma = frexp(amax, &ea), mb = frexp(bmax, &eb);
-    // the mantissas rounded up to float: the bound stays an upper bound
-    o[3] = make_int4(__float_as_int(__double2float_ru(ma)), ea,
-                     __float_as_int(__double2float_ru(mb)), eb);
-    o[4] = make_int4(__float_as_int(__double2float_ru(z2max)), k, 0, 0);
+    if (Rm.x == 0. && Rm.y == 0.) eR = FE_ZERO_E;
+    // the bound's mantissa rounded up to float: it stays an upper bound
+    const float ma = __double2float_ru(frexp(amax, &ea));
+    const int Rx = __float_as_int((float)Rm.x), Ry = __float_as_int((float)Rm.y);
+    const int eQ = __shfl_xor_sync(am, eP, 1), rx = __shfl_xor_sync(am, Rx, 1),
+              ry = __shfl_xor_sync(am, Ry, 1), er = __shfl_xor_sync(am, eR, 1),
+              mb = __shfl_xor_sync(am, __float_as_int(ma), 1), eb = __shfl_xor_sync(am, ea, 1);
+    if (!ok) {
+        if (!odd) o[4] = make_int4(0, 0, 0, 0);
+    } else if (!odd) {
+        o[0] = runs_pack2(P, eP, eQ);
+        o[3] = make_int4(__float_as_int(ma), ea, mb, eb);
+        o[4] = make_int4(__float_as_int(__double2float_ru(z2max)), k, 0, 0);
+    } else {
+        o[1] = make_int4(__float_as_int((float)P.x), __float_as_int((float)P.y), rx, ry);
+        o[2] = make_int4(er, eR, Rx, Ry);
+    }
 }
 
 __global__ void k_fe_path(const double2 *std_p, const double2 *xm, const int *xe, int n,
@@ -980,30 +982,21 @@ void fsg_build_bla(const RefDev *Rd, int flavor, int len, double2 *M2, double *M
 
 void fsg_build_fe_runs(const RefDev *Rd, int len, const int4 *Zp, const int4 *Df, int4 *runs,
                        cudaStream_t s) {
-    const int tb = 128;
-    k_fe_runs<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Rd, Zp, Df, len, runs);
+    const int tb = 64;
+    k_fe_runs<<<(2 * (len + 1) + tb - 1) / tb, tb, 0, s>>>(Rd, Zp, Df, len, runs);
 }
-void fsg_build_plain_orbit(const RefDev *Rd, int len, const int4 *Zf, int4 *Zp, cudaStream_t s) {
-    int tb = 256;
+void fsg_build_fe_orbit(const RefDev *Rd, int len, int4 *Zf, int4 *Zp, cudaStream_t s) {
+    const int tb = 256;
+    k_fe_orbit<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Rd, Zf);
     k_plain_orbit<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Rd, Zf, Zp);
 }
-
-void fsg_build_fe_bla(const RefDev *Rd, const double2 *Mbla, const double *rbla, int bla_len,
-                      int4 *bla_f, int bla_nit, int4 *bla_first, int *bla_first_step,
-                      double kc, int4 *bla_chain, int2 *bla_chain_step, cudaStream_t s);
-
-void fsg_build_fe_tables(const RefDev *Rd, int len, int4 *Zf, const double2 *dzndc,
-                         const double2 *dzndc_xm, const int *dzndc_xe, int4 *dzndc_f,
-                         const double2 *dzndz, const double2 *dzndz_xm, const int *dzndz_xe,
-                         int4 *dzndz_f, const double2 *Mbla, const double *rbla, int bla_len,
-                         int4 *bla_f, int bla_nit, int4 *bla_first, int *bla_first_step,
-                         double kc, int4 *bla_chain, int2 *bla_chain_step, cudaStream_t s) {
-    int tb = 256;
-    k_fe_orbit<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Rd, Zf);
+void fsg_build_fe_paths(int len, const double2 *dzndc, const double2 *dzndc_xm,
+                        const int *dzndc_xe, int4 *dzndc_f, const double2 *dzndz,
+                        const double2 *dzndz_xm, const int *dzndz_xe, int4 *dzndz_f,
+                        cudaStream_t s) {
+    const int tb = 256;
     if (dzndc_f) k_fe_path<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(dzndc, dzndc_xm, dzndc_xe, len + 1, dzndc_f);
     if (dzndz_f) k_fe_path<<<(len + 2 + tb - 1) / tb, tb, 0, s>>>(dzndz, dzndz_xm, dzndz_xe, len + 2, dzndz_f);
-    fsg_build_fe_bla(Rd, Mbla, rbla, bla_len, bla_f, bla_nit, bla_first, bla_first_step, kc,
-                     bla_chain, bla_chain_step, s);
 }
 
 void fsg_build_fe_bla(const RefDev *Rd, const double2 *Mbla, const double *rbla, int bla_len,

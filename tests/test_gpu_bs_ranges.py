@@ -57,3 +57,42 @@ def test_bs_fp64_ranges_vs_oracle(ctx, flavor, seed, width, hess):
     assert np.array_equal(k, ~np.isnan(Z))
     # bit for bit, but for the sign of a zero
     assert np.array_equal(Z[k], Zo[:Z.shape[0]][k])
+
+
+@pytest.mark.parametrize("hess", [True, False])
+@pytest.mark.parametrize("width", ["1e-5", "1e-30", "1e-200", "1e-320"])
+@pytest.mark.parametrize("mode", ["fe32", "fp64"])
+def test_bs_real_reference_alone_and_in_a_mixed_launch(ctx, mode, width, hess):
+    """A launch whose references are all real takes the kernel of the real
+    axis; in one launch with a reference off it, the general one: the same
+    pixels bit for bit."""
+    import mpmath
+    from fractalshades_gb300 import _native as nat
+    if mode == "fp64" and width == "1e-320":
+        pytest.skip("below the double form's range")
+    dx = fsx.mpf_to_Xrange(mpmath.mpf(width))
+    kc = float(np.ldexp(dx.m, dx.e))
+    xs, ys = syn.image_axes(37, 29)
+    n = xs.size * ys.size
+    refs = []
+    for seed in (4, 5):                                  # on the real axis, off it
+        t = syn.config4_workload(seed=seed, n_tiles=1, max_iter=600, kind=1)[0]
+        refs.append(nat.Reference(ctx, t.Zn, div_iter=t.div_iter, order=t.ref_order, flavor=1,
+                                  calc_dzndc=hess, scale_m=dx.m, scale_e=dx.e, bla=True, kc=kc,
+                                  bla_eps=1e-6))
+
+    def run(which):
+        out, tiles = [], []
+        for k in which:
+            o = (np.zeros((6 if hess else 2, n)), -np.ones((1, n), dtype=np.int8),
+                 np.zeros((1, n), dtype=np.int32))
+            out.append(o)
+            tiles.append(nat.make_tile(xs=xs, ys=ys, lin_mat=LIN, Z=o[0], stop_reason=o[1],
+                                       stop_iter=o[2], ref=refs[k], dx_m=dx.m, dx_e=dx.e,
+                                       drift_m=0.01 * dx.m, drift_e=dx.e, drifty_m=0., drifty_e=0))
+        ctx.perturb_tiles(nat.make_calc(max_iter=3000, M_divergence=1000., flavor=1, calc_dzndc=hess,
+                                        bla=True, mode=mode), tiles)
+        return out
+
+    for a, b in zip(run([0])[0], run([0, 1])[0]):
+        assert np.array_equal(a, b, equal_nan=a.dtype == np.float64)
