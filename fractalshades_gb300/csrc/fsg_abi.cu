@@ -96,12 +96,16 @@ struct fsg_ctx {
     char *scratch = nullptr; size_t scratch_size = 0;
     // grow-only device scratch of the longest-first claim order
     char *lpt = nullptr; size_t lpt_size = 0;
+    // memory of the reference tables (ref_pool)
+    cudaMemPool_t ref_pool = nullptr; bool ref_pool_asked = false;
 };
 
 struct fsg_ref {
     RefDev host;            // device pointers, host copy
     RefDev *dev = nullptr;  // device copy of the descriptor
-    std::vector<void *> allocs;   // stream-ordered allocations (cudaMallocAsync)
+    std::vector<void *> allocs;   // stream-ordered allocations
+    char *block = nullptr;        // free rest of the block small tables are carved from
+    size_t block_left = 0;
     int64_t len = 0;
     int xr_paths = 0, flavor = 0, has_dzndc = 0, has_dzndz = 0;
     int nexp = 0;                 // 0: power-2 model, n: power-n model
@@ -132,13 +136,67 @@ int cuda_err(fsg_ctx *c, cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return cuda_err(ctx, e_, what); \
     } while (0)
 
+// The pool a context's reference tables come from.  The device's default pool
+// unmaps what is free at every synchronisation, and building and freeing a
+// reference both synchronise: a program that builds one per view mapped its
+// tables anew each time, 0.18 ms of the 1.18 ms of a new 256 x 256 view.  This pool
+// keeps up to FSG_REF_POOL_KEEP free bytes, belongs to the context and goes with
+// it (memory of references that outlive the context is given back when they
+// are freed); the driver orders reuse between streams.
+#define FSG_REF_POOL_KEEP (32ull << 20)
+cudaMemPool_t ref_pool(fsg_ctx *ctx) {
+    if (ctx->ref_pool_asked) return ctx->ref_pool;
+    ctx->ref_pool_asked = true;
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    unsigned long long keep = FSG_REF_POOL_KEEP;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        cudaMemPoolDestroy(pool);
+        return nullptr;
+    }
+    return ctx->ref_pool = pool;
+}
+
+cudaError_t ref_malloc(fsg_ctx *ctx, void **p, size_t bytes) {
+    cudaMemPool_t pool = ref_pool(ctx);
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, ctx->stream)
+                : cudaMallocAsync(p, bytes, ctx->stream);
+}
+
 template <class T>
 int ref_alloc(fsg_ctx *ctx, fsg_ref *r, T **p, size_t n) {
+    // A reference has some twenty tables; an allocation costs about 2 us of
+    // host time, so those of a small orbit share blocks of at most 1 MiB
+    // (256 B a point, about two thirds of what a point's tables take); a table
+    // larger than a quarter of the block is allocated by itself.
+    const size_t bytes = (n * sizeof(T) + 16 + 255) & ~(size_t)255;
+    size_t blk = 256 * (size_t)r->len;
+    if (blk > (1u << 20)) blk = 1u << 20;
     void *q = nullptr;
-    // stream-ordered: no device-wide synchronisation while other streams run
-    cudaError_t e = cudaMallocAsync(&q, n * sizeof(T) + 16, ctx->stream);
-    if (e != cudaSuccess) return cuda_err(ctx, e, "cudaMalloc(reference table)");
-    r->allocs.push_back(q);
+    if (bytes > r->block_left || bytes > blk / 4) {
+        // stream-ordered: no device-wide synchronisation while other streams run
+        const bool own = bytes > blk / 4;
+        cudaError_t e = ref_malloc(ctx, &q, own ? bytes : blk);
+        if (e != cudaSuccess) return cuda_err(ctx, e, "cudaMalloc(reference table)");
+        r->allocs.push_back(q);
+        if (!own) {
+            r->block = (char *)q + bytes;
+            r->block_left = blk - bytes;
+        }
+    } else {
+        q = r->block;
+        r->block += bytes;
+        r->block_left -= bytes;
+    }
     *p = (T *)q;
     return FSG_OK;
 }
@@ -784,6 +842,7 @@ int fsg_ctx_destroy(fsg_ctx *ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->lpt) cudaFree(ctx->lpt);
+    if (ctx->ref_pool) cudaMemPoolDestroy(ctx->ref_pool);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     if (ctx->used_dev) cudaFree(ctx->used_dev);
     if (ctx->counter_dev) cudaFree(ctx->counter_dev);
@@ -989,27 +1048,21 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
     }
     R.bs_Zf = bs_Zf; R.bs_hf = bs_hf; R.bs_blaf = bs_blaf; R.bs_rf = bs_rf;
     R.bs_fa = bs_fa; R.bs_fz = bs_fz; R.bs_fh = bs_fh;
-    RCK(cudaMallocAsync((void **)&r->dev, sizeof(RefDev), s), "cudaMallocAsync(reference descriptor)");
+    RCK(ref_malloc(ctx, (void **)&r->dev, sizeof(RefDev)), "cudaMallocAsync(reference descriptor)");
     RCK(cudaMemcpyAsync(r->dev, &R, sizeof(RefDev), cudaMemcpyHostToDevice, s), "upload descriptor");
     // Builds.  The derivative paths are serial walks of one block; what needs
     // only the orbit (the BLA tree, the fe orbit and BLA tables) runs beside
     // them on the copy stream, which is idle between calls, and the context
     // stream takes both up again before the tables that need a path.  A 2474
     // point reference with its path and tree: 0.73 ms on one stream, 0.58 ms
-    // on two (0.55 of it the walk).  With no path to walk, one stream.
+    // on two (0.55 of it the walk, which is therefore launched first).  With no
+    // path to walk, one stream.
     const bool forked = R.bla_len > 0 && (d->calc_dzndc || (d->flavor == 0 && d->calc_dzndz));
     cudaStream_t side = forked ? ctx->copy_stream : s;
     if (forked) {
         RCK(cudaEventRecord(ctx->ev_seg[0], s), "cudaEventRecord(reference)");
         RCK(cudaStreamWaitEvent(side, ctx->ev_seg[0], 0), "cudaStreamWaitEvent(reference)");
     }
-    if (R.bla_len > 0) fsg_build_bla(r->dev, d->flavor, len, Mbla, Mbs, rbla, stages, d->kc, d->bla_eps, side);
-    if (fe_tables) {
-        fsg_build_fe_orbit(r->dev, len, Zf, Zp, side);
-        fsg_build_fe_bla(r->dev, Mbla, rbla, R.bla_len, bla_f, bla_nit, bla_first, bla_first_step,
-                         d->kc, bla_chain, bla_chain_step, side);
-    }
-    if (d->flavor != 0) fsg_build_bs_fr_bla(Mbs, rbla, R.bla_len, bs_blaf, bs_rf, side);
     if (d->flavor == 0) {
         fsg_build_paths_m2(r->dev, len, dzndc, dzndc_xm, dzndc_xe, dzndz, dzndz_xm, dzndz_xe,
                            R.div_iter, d->xr_paths, d->calc_dzndc, d->calc_dzndz, d->scale_m,
@@ -1018,6 +1071,13 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
         fsg_build_paths_bs(r->dev, len, dXa, dXb, dYa, dYb, ldexp(d->scale_m, d->scale_e), s);
         if (bs_xpm) fsg_build_paths_bs_xr(r->dev, len, bs_xpm, bs_xpe, d->scale_m, d->scale_e, s);
     }
+    if (R.bla_len > 0) fsg_build_bla(r->dev, d->flavor, len, Mbla, Mbs, rbla, stages, d->kc, d->bla_eps, side);
+    if (fe_tables) {
+        fsg_build_fe_orbit(r->dev, len, Zf, Zp, side);
+        fsg_build_fe_bla(r->dev, Mbla, rbla, R.bla_len, bla_f, bla_nit, bla_first, bla_first_step,
+                         d->kc, bla_chain, bla_chain_step, side);
+    }
+    if (d->flavor != 0) fsg_build_bs_fr_bla(Mbs, rbla, R.bla_len, bs_blaf, bs_rf, side);
     if (forked) {
         // nothing may be released while the side stream still writes it: an
         // event that cannot be had is replaced by a wait on the host
@@ -1105,7 +1165,7 @@ int fsg_ref_derive_bla(fsg_ctx *ctx, fsg_ref *base, double kc, double bla_eps, f
     R.Mbla = Mbla; R.Mbla_bs = Mbs; R.rbla = rbla; R.bs_blaf = bs_blaf; R.bs_rf = bs_rf;
     R.bla_f = bla_f; R.bla_first = bla_first; R.bla_first_step = bla_first_step;
     R.bla_chain = bla_chain; R.bla_chain_step = bla_chain_step;
-    RCK(cudaMallocAsync((void **)&r->dev, sizeof(RefDev), s), "cudaMallocAsync(reference descriptor)");
+    RCK(ref_malloc(ctx, (void **)&r->dev, sizeof(RefDev)), "cudaMallocAsync(reference descriptor)");
     RCK(cudaMemcpyAsync(r->dev, &R, sizeof(RefDev), cudaMemcpyHostToDevice, s), "upload descriptor");
     if (R.bla_len > 0) {
         fsg_build_bla(r->dev, R.flavor, len, Mbla, Mbs, rbla, R.stages, kc, bla_eps, s);
