@@ -1054,8 +1054,8 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
     // only the orbit (the BLA tree, the fe orbit and BLA tables) runs beside
     // them on the copy stream, which is idle between calls, and the context
     // stream takes both up again before the tables that need a path.  A 2474
-    // point reference with its path and tree: 0.73 ms on one stream, 0.58 ms
-    // on two (0.55 of it the walk, which is therefore launched first).  With no
+    // point reference with its path and tree: 0.57 ms on one stream, 0.42 ms
+    // on two (0.39 of it the walk, which is therefore launched first).  With no
     // path to walk, one stream.
     const bool forked = R.bla_len > 0 && (d->calc_dzndc || (d->flavor == 0 && d->calc_dzndz));
     cudaStream_t side = forked ? ctx->copy_stream : s;

@@ -30,21 +30,36 @@ __device__ __forceinline__ xc orbit_xr(const RefDev &R, int i) {
 // Sequential form (orbits up to FSG_PATH_SCAN_MIN = 8192 points), in the
 // reference's order: D_i = a_i D_{i-1} (+ s), a_i = df/dz(Z_{i-1}).  The chain of
 // one step after the other is all of the time: an FP64 instruction returns after
-// 63 clocks, its result reaches an integer test after 40 more, a vote or a
-// shuffle takes 30 and a taken branch 20.  Two lanes walk the chain, one for
-// each part of D: two products, their sum, the sum with s, and the parts change
-// hands.  The Xrange tests are read every FSG_PATH_RUN steps; steps that ask for
-// more than the chain does are taken again.  The block's threads turn
-// FSG_PATH_PART orbit points at a time into a_i in shared memory, and write the
-// part's results.  2474 points, Xrange: 1.80 ms with one thread doing everything,
-// 0.55 ms like this.  The paths are zero-filled by the host (cudaMemsetAsync)
-// before the launch.
+// 63 clocks and the next of its warp can start 78 after it, its result reaches a
+// shuffle or an integer test after 40 more, a vote or a shuffle takes 30 and a
+// taken branch 20.  So four lanes walk the chain, one for each real product of a
+// step: every lane multiplies once, takes its partner's product and adds, which
+// leaves it with the part that its next product asks for:
+//   lane            0        1        2        3
+//   holds           D.x      D.x      D.y      D.y
+//   product         a.x D.x  a.y D.x  a.x D.y  -a.y D.y
+//   sum with lane   3: D'.x  2: D'.y  1: D'.y  0: D'.x
+// and in every second step lanes 1 and 3 stand for each other.  The sum with s
+// is left out where s is below half an ulp of the real part, as it is once the
+// derivative has grown: a run without it looks whether that held and is taken
+// again with it where it did not.  A warp issues in order, so whatever stands
+// between two links of the chain delays it: the coefficients of a run are read
+// while the one before it is on its way, and the Xrange tests and the stores
+// follow the FSG_PATH_RUN steps; steps that ask for more than the chain does are
+// taken again.  The block's threads turn FSG_PATH_PART orbit points at a time into
+// a_i in shared memory, and write the part's results.  2474 points, Xrange: 1.80 ms
+// with one thread doing everything, 0.55 ms with a lane for each part of D and the
+// tests between the steps, 0.39 ms like this.  The paths are zero-filled by
+// the host (cudaMemsetAsync) before the launch.
 #define FSG_PATH_PART 256
 #define FSG_PATH_THREADS 128
-#define FSG_PATH_RUN 8          // steps between two looks at the Xrange tests
+#define FSG_PATH_RUN 16         // steps between two looks at the Xrange tests
+#define FSG_PATH_LIM (FSG_PATH_PART / 32)
 struct PathShared {
     double2 a[FSG_PATH_PART], out[FSG_PATH_PART];
-    int ae[FSG_PATH_PART], oe[FSG_PATH_PART];
+    int ae[FSG_PATH_PART], oe[FSG_PATH_PART];   // exponents of a_i and of D_i
+    double c[FSG_PATH_PART][4], u[FSG_PATH_PART][4];    // what the four lanes multiply by and add
+    int4 lim[FSG_PATH_PART / FSG_PATH_LIM];     // of FSG_PATH_LIM steps each (path_prep)
 };
 
 // xr_add(xr_mul(a 2^ae, D), s 2^se), or caddr(cmul(a, D), s)
@@ -58,16 +73,109 @@ static __device__ __noinline__ xc path_step_full(double2 a, int ae, xc D, double
     return affine ? xr_add(r, xc_make(s, 0., se)) : r;
 }
 
+// the exponent of a_k in the scan (a larger one is not for the chain: no sum of
+// them overflows)
+__device__ __forceinline__ int path_ae(const PathShared &S, int k) {
+    return max(min(S.ae[k], 100000), -100000);
+}
+// Coefficients, addends and exponents of the steps [k0, cnt) of a part from D's
+// exponent e, for the chain (one warp).  Xrange: without a renormalisation D's
+// exponent is e_k = max(e_{k-1} + ae_k, se) (the sum with s takes the larger of
+// the two; s = 0 in the path without one), a scan over the lanes' 8 steps each;
+// the product's share of the shift to e_k goes to a (a power of two: the same
+// bits while nothing leaves the normal range).  lim: of FSG_PATH_LIM steps the smallest shift,
+// the largest field of the addend, and whether one is not for the chain.
+template <bool XR, bool AFFINE>
+__device__ __forceinline__ void path_prep(PathShared &S, int k0, int cnt, int e, double s, int se) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, b = k0 + lane * FSG_PATH_LIM, b1 = min(b + FSG_PATH_LIM, cnt);
+    if (XR) {
+        const int none = -(1 << 30);
+        int sum = 0, top = none;                 // e -> max(e + sum, top)
+        for (int k = b; k < b1; k++) {
+            const int x = path_ae(S, k);
+            sum += x;
+            top = max(top + x, se);
+        }
+        for (int d = 1; d < 32; d <<= 1) {
+            const int s1 = __shfl_up_sync(all, sum, d), t1 = __shfl_up_sync(all, top, d);
+            if (lane >= d) { top = max(t1 + sum, top); sum += s1; }
+        }
+        const int s1 = __shfl_up_sync(all, sum, 1), t1 = __shfl_up_sync(all, top, 1);
+        if (lane > 0) e = AFFINE ? max(e + s1, t1) : e + s1;
+    }
+    int4 lim = make_int4(0, 0, 0, 0);
+    for (int k = b; k < b1; k++) {
+        const double2 a = S.a[k];
+        double x = a.x, y = a.y, u = AFFINE ? s : 0.;
+        if (XR) {
+            const int e1 = e + path_ae(S, k), t = AFFINE ? min(e1 - se, 0) : 0;
+            x = xr_exp2_shift(x, t);
+            y = xr_exp2_shift(y, t);
+            if (AFFINE) u = xr_exp2_shift(s, min(se - e1, 0));
+            // not for the chain: what the shift does not cover, and a zero part of
+            // a, where xr_mul renormalises
+            lim.z |= (t < -800) | (path_ae(S, k) != S.ae[k]) | (d_field_min(a) == 0);
+            lim.x = min(lim.x, t);
+            S.oe[k] = e = AFFINE ? max(e1, se) : e1;
+        }
+        lim.y = max(lim.y, d_field(u));
+        const double ny = d_flip(y, 0x80000000u);
+        const bool second = k & 1;
+        S.c[k][0] = x; S.c[k][1] = second ? ny : y;
+        S.c[k][2] = x; S.c[k][3] = second ? y : ny;
+        S.u[k][0] = u; S.u[k][1] = second ? u : 0.;
+        S.u[k][2] = 0.; S.u[k][3] = second ? 0. : u;
+    }
+    if (b < b1) S.lim[b / FSG_PATH_LIM] = lim;
+    __syncwarp();
+}
+
+// FSG_PATH_RUN steps of the chain; ADD: with the sums.  odd: a product asks for
+// xr_mul's lazy renormalisation (of the product before the shift: looked at with
+// the run's smallest shift), or has a zero part; far: every addend was below half an ulp (55 binary orders, and one for a
+// power of two; nor is the other part a zero, whose sum with 0 may change its
+// sign)
+template <bool XR, bool AFFINE, bool ADD>
+__device__ __forceinline__ void path_run(const double (&c)[FSG_PATH_RUN], const double (&u)[FSG_PATH_RUN],
+                                         PathShared &S, int k0, int4 lim, double &own, bool &odd,
+                                         bool &far) {
+    double m[FSG_PATH_RUN], o[FSG_PATH_RUN];
+#pragma unroll
+    for (int j = 0; j < FSG_PATH_RUN; j++) {
+        const double p = d_mul_here(c[j], own);
+        m[j] = d_add_here(p, __shfl_xor_sync(0xffffffffu, p, (j & 1) ? 1 : 3));
+        own = ADD ? d_add_here(m[j], u[j]) : m[j];
+        o[j] = own;
+    }
+    // (lane 0 always ends on the real part, lane 2 on the imaginary one)
+    if (threadIdx.x == 0 || threadIdx.x == 2) {
+#pragma unroll
+        for (int j = 0; j < FSG_PATH_RUN; j++) ((double *)&S.out[k0 + j])[threadIdx.x >> 1] = o[j];
+    }
+    unsigned lo = ~0u, hi = 0u;              // of the words without their signs
+#pragma unroll
+    for (int j = 0; j < FSG_PATH_RUN; j++) {
+        const unsigned w = d_hi(m[j]) << 1;
+        lo = min(lo, w);
+        hi = max(hi, w);
+    }
+    const int l = (int)(lo >> 21), h = (int)(hi >> 21);
+    if (XR) odd |= (l < 923) | (h - lim.x > 1123);
+    far = l - lim.y >= 56;
+}
+
 // indices [first, valid) from prev at first - 1; returns the last value (warp 0)
 template <bool XR, bool AFFINE>
 __device__ __forceinline__ xc path_seq(const RefDev &R, PathShared &S, int first, int valid, xc prev,
                                        double s, int se, double2 *__restrict__ out_std,
                                        double2 *__restrict__ out_xm, int *__restrict__ out_xe) {
-    const int role = threadIdx.x & 1;                // 0: real part, 1: imaginary
-    const unsigned minus = role ? 0u : 0x80000000u;
-    const bool s0 = AFFINE && d_is0(s);
-    double own = role ? prev.im : prev.re, oth = role ? prev.re : prev.im;
-    int e = prev.e;
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 3;
+    const bool s0 = XR && AFFINE && d_is0(s);
+    double own = (lane & 2) ? prev.im : prev.re;
+    int e = prev.e;                         // D's exponent ahead of the part
+    bool skip = false;                      // the next run is tried without the sums
     for (int base = first; base < valid; base += FSG_PATH_PART) {
         const int cnt = min(FSG_PATH_PART, valid - base);
         for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
@@ -82,61 +190,64 @@ __device__ __forceinline__ xc path_seq(const RefDev &R, PathShared &S, int first
         }
         __syncthreads();
         if (threadIdx.x < 32) {
+            path_prep<XR, AFFINE>(S, 0, cnt, e, s, se);
+            double c1[FSG_PATH_RUN], u1[FSG_PATH_RUN];
+            int4 lim1 = make_int4(0, 0, 1, 0);
+            auto fetch = [&](int k0) {      // the run from k0
+                lim1.z = 1;
+                if (k0 + FSG_PATH_RUN > cnt) return;
+#pragma unroll
+                for (int j = 0; j < FSG_PATH_RUN; j++) { c1[j] = S.c[k0 + j][lane]; u1[j] = S.u[k0 + j][lane]; }
+                lim1 = make_int4(0, 0, s0, 0);
+#pragma unroll
+                for (int j = 0; j < FSG_PATH_RUN; j += FSG_PATH_LIM) {
+                    const int4 x = S.lim[(k0 + j) / FSG_PATH_LIM];
+                    lim1 = make_int4(min(lim1.x, x.x), max(lim1.y, x.y), lim1.z | x.z, 0);
+                }
+            };
+            fetch(0);
             for (int k0 = 0; k0 < cnt; k0 += FSG_PATH_RUN) {
-                const int k1 = min(k0 + FSG_PATH_RUN, cnt);
-                const double own0 = own, oth0 = oth;
-                const int e0 = e;
-                bool odd = k1 - k0 < FSG_PATH_RUN;
-                double2 as[FSG_PATH_RUN];
-                int es[FSG_PATH_RUN];
+                const double own0 = own;
+                const int4 lim = lim1;
+                bool odd = lim.z != 0;
+                double c[FSG_PATH_RUN], u[FSG_PATH_RUN];
+#pragma unroll
+                for (int j = 0; j < FSG_PATH_RUN; j++) { c[j] = c1[j]; u[j] = u1[j]; }
+                fetch(k0 + FSG_PATH_RUN);
                 if (!odd) {
-#pragma unroll
-                    for (int j = 0; j < FSG_PATH_RUN; j++) { as[j] = S.a[k0 + j]; es[j] = S.ae[k0 + j]; }
-                }
-#pragma unroll
-                for (int j = 0; j < FSG_PATH_RUN; j++) {
-                    if (odd && j == 0) break;
-                    const int k = k0 + j;
-                    const double2 a = as[j];
-                    if (XR) {
-                        // xr_add takes D's product and s on the larger of their
-                        // exponents; the product's share of that shift goes to a,
-                        // ahead of the chain (a power of two: the same bits while
-                        // nothing leaves the normal range)
-                        const int e1 = (int)((unsigned)e + (unsigned)es[j]);
-                        const int t = AFFINE ? min(e1 - se, 0) : 0;
-                        const double u = role || !AFFINE ? 0. : xr_exp2_shift(s, min(se - e1, 0));
-                        const double m = xr_exp2_shift(a.x, t) * own
-                                         + xr_exp2_shift(d_flip(a.y, minus), t) * oth;
-                        own = AFFINE ? m + u : m;
-                        e = AFFINE ? max(e1, se) : e1;
-                        // xr_mul's lazy renormalisation (of the product before the
-                        // shift; a zero part asks for it too), and what the shift
-                        // does not cover
-                        odd |= ((unsigned)(d_field(m) - t - 923) > 200u) | (t < -800) | s0
-                               | (d_field_min(a) == 0);
-                        if (threadIdx.x == 0) S.oe[k] = e;
-                    } else {
-                        // cmul(a, D): a.x D.x - a.y D.y, a.x D.y + a.y D.x
-                        const double m = a.x * own + d_flip(a.y, minus) * oth;
-                        own = AFFINE ? m + (role ? 0. : s) : m;
+                    bool far;
+                    if (!AFFINE || skip) {
+                        path_run<XR, AFFINE, false>(c, u, S, k0, lim, own, odd, far);
+                        odd = __any_sync(all, odd | (AFFINE && !far));
+                        skip = !odd;
                     }
-                    oth = __shfl_xor_sync(0xffffffffu, own, 1);
-                    if (threadIdx.x < 2) ((double *)&S.out[k])[role] = own;
+                    if (AFFINE && !skip) {
+                        own = own0; odd = false;
+                        path_run<XR, AFFINE, true>(c, u, S, k0, lim, own, odd, far);
+                        odd = __any_sync(all, odd);
+                        skip = __all_sync(all, far) && !odd;
+                    }
                 }
-                if (__any_sync(0xffffffffu, odd)) {
+                if (odd) {
                     // these steps again (and what is left of the part), with the
                     // reference's operations
-                    xc r = role ? xc_make(oth0, own0, e0) : xc_make(own0, oth0, e0);
+                    const int k1 = min(k0 + FSG_PATH_RUN, cnt), was = XR ? S.oe[k1 - 1] : 0;
+                    xc r = xc_make(__shfl_sync(all, own0, 0), __shfl_sync(all, own0, 2),
+                                   k0 > 0 && XR ? S.oe[k0 - 1] : e);
                     for (int k = k0; k < k1; k++) {
                         r = path_step_full<XR>(S.a[k], S.ae[k], r, s, se, AFFINE);
+                        __syncwarp();
                         if (threadIdx.x == 0) { S.out[k] = xm(r); S.oe[k] = r.e; }
                     }
-                    own = role ? r.im : r.re;
-                    oth = role ? r.re : r.im;
-                    e = r.e;
+                    __syncwarp();
+                    own = (lane & 2) ? r.im : r.re;
+                    if (XR && r.e != was && k1 < cnt) {
+                        path_prep<XR, AFFINE>(S, k1, cnt, r.e, s, se);
+                        fetch(k1);
+                    }
                 }
             }
+            if (XR) e = S.oe[cnt - 1];
         }
         __syncthreads();
         for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
@@ -146,7 +257,7 @@ __device__ __forceinline__ xc path_seq(const RefDev &R, PathShared &S, int first
         // (the next part's values overwrite these)
         __syncthreads();
     }
-    return xc_make(role ? oth : own, role ? own : oth, e);
+    return xc_make(__shfl_sync(all, own, 0), __shfl_sync(all, own, 2), e);
 }
 
 template <bool XR>
