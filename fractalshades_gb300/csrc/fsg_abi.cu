@@ -39,9 +39,7 @@ void fsg_build_fe_paths(int len, const double2 *dzndc, const double2 *dzndc_xm,
                         const double2 *dzndz_xm, const int *dzndz_xe, int4 *dzndz_f,
                         cudaStream_t s);
 void fsg_build_fe_bla(const RefDev *Rd, const double2 *Mbla, const double *rbla, int bla_len,
-                      int4 *bla_f, int bla_nit, int4 *bla_first, int *bla_first_step,
-                      double kc, int4 *bla_chain, int2 *bla_chain_step,
-                      cudaStream_t s);
+                      int4 *bla_f, int bla_nit, int4 *bla_at, double kc, cudaStream_t s);
 void fsg_build_bs_fr(const RefDev *Rd, int len, int4 *Zf, const double *dXa, const double *dXb,
                      const double *dYa, const double *dYb, int4 *hf, float4 *fa, int4 *fz,
                      float4 *fh, int div_iter, cudaStream_t s);
@@ -1005,9 +1003,7 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
     R.Mbla = Mbla; R.Mbla_bs = Mbs; R.rbla = rbla; R.stages = stages;
     // fe tables (M2)
     int4 *Zf = nullptr, *Zp = nullptr, *dzndc_f = nullptr, *dzndz_f = nullptr, *bla_f = nullptr,
-         *bla_first = nullptr, *bla_chain = nullptr, *fe_runs = nullptr;
-    int *bla_first_step = nullptr;
-    int2 *bla_chain_step = nullptr;
+         *bla_at = nullptr, *fe_runs = nullptr;
     const int bla_nit = (len >> 3) + 1;
     const bool fe_tables = d->flavor == 0 && d->nexp == 0;   // FE32 is the power-2 form
     if (fe_tables) {
@@ -1018,15 +1014,11 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
         if (d->calc_dzndz) RA(dzndz_f, len + 2);
         if (R.bla_len > 0) {
             RA(bla_f, 2 * (size_t)R.bla_len);
-            RA(bla_first, 2 * (size_t)bla_nit);
-            RA(bla_first_step, (size_t)bla_nit);
-            RA(bla_chain, 2 * (size_t)bla_nit);
-            RA(bla_chain_step, (size_t)bla_nit);
+            RA(bla_at, 5 * (size_t)bla_nit);
         }
     }
     R.Zf = Zf; R.Zp = Zp; R.dZndc_f = dzndc_f; R.dZndz_f = dzndz_f; R.bla_f = bla_f;
-    R.bla_first = bla_first; R.bla_first_step = bla_first_step; R.bla_nit = bla_nit;
-    R.bla_chain = bla_chain; R.bla_chain_step = bla_chain_step;
+    R.bla_at = bla_at; R.bla_nit = bla_nit;
     R.fe_runs = fe_runs;
     // FP32+exp tables (Burning Ship)
     int4 *bs_Zf = nullptr, *bs_hf = nullptr, *bs_blaf = nullptr;
@@ -1074,8 +1066,7 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
     if (R.bla_len > 0) fsg_build_bla(r->dev, d->flavor, len, Mbla, Mbs, rbla, stages, d->kc, d->bla_eps, side);
     if (fe_tables) {
         fsg_build_fe_orbit(r->dev, len, Zf, Zp, side);
-        fsg_build_fe_bla(r->dev, Mbla, rbla, R.bla_len, bla_f, bla_nit, bla_first, bla_first_step,
-                         d->kc, bla_chain, bla_chain_step, side);
+        fsg_build_fe_bla(r->dev, Mbla, rbla, R.bla_len, bla_f, bla_nit, bla_at, d->kc, side);
     }
     if (d->flavor != 0) fsg_build_bs_fr_bla(Mbs, rbla, R.bla_len, bs_blaf, bs_rf, side);
     if (forked) {
@@ -1137,9 +1128,7 @@ int fsg_ref_derive_bla(fsg_ctx *ctx, fsg_ref *base, double kc, double bla_eps, f
 #define RA(ptr, n) do { rc = ref_alloc(ctx, r, &(ptr), (n)); if (rc != FSG_OK) { ref_release(r, s); delete r; return rc; } } while (0)
 #define RCK(call, what) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { ref_release(r, s); delete r; return cuda_err(ctx, e_, what); } } while (0)
     double2 *Mbla = nullptr; double *Mbs = nullptr, *rbla = nullptr;
-    int4 *bla_f = nullptr, *bla_first = nullptr, *bla_chain = nullptr;
-    int *bla_first_step = nullptr;
-    int2 *bla_chain_step = nullptr;
+    int4 *bla_f = nullptr, *bla_at = nullptr;
     R.bla_len = 0;
     if (L > 0) {
         if (R.flavor == 0) RA(Mbla, 4 * (size_t)L); else RA(Mbs, 16 * (size_t)L);
@@ -1150,10 +1139,7 @@ int fsg_ref_derive_bla(fsg_ctx *ctx, fsg_ref *base, double kc, double bla_eps, f
         R.bla_len = 2 * L;
         if (R.flavor == 0 && R.nexp == 0) {
             RA(bla_f, 2 * (size_t)R.bla_len);
-            RA(bla_first, 2 * (size_t)R.bla_nit);
-            RA(bla_first_step, (size_t)R.bla_nit);
-            RA(bla_chain, 2 * (size_t)R.bla_nit);
-            RA(bla_chain_step, (size_t)R.bla_nit);
+            RA(bla_at, 5 * (size_t)R.bla_nit);
         }
     }
     int4 *bs_blaf = nullptr;
@@ -1163,15 +1149,13 @@ int fsg_ref_derive_bla(fsg_ctx *ctx, fsg_ref *base, double kc, double bla_eps, f
         RA(bs_rf, (size_t)R.bla_len);
     }
     R.Mbla = Mbla; R.Mbla_bs = Mbs; R.rbla = rbla; R.bs_blaf = bs_blaf; R.bs_rf = bs_rf;
-    R.bla_f = bla_f; R.bla_first = bla_first; R.bla_first_step = bla_first_step;
-    R.bla_chain = bla_chain; R.bla_chain_step = bla_chain_step;
+    R.bla_f = bla_f; R.bla_at = bla_at;
     RCK(ref_malloc(ctx, (void **)&r->dev, sizeof(RefDev)), "cudaMallocAsync(reference descriptor)");
     RCK(cudaMemcpyAsync(r->dev, &R, sizeof(RefDev), cudaMemcpyHostToDevice, s), "upload descriptor");
     if (R.bla_len > 0) {
         fsg_build_bla(r->dev, R.flavor, len, Mbla, Mbs, rbla, R.stages, kc, bla_eps, s);
         if (R.flavor == 0 && R.nexp == 0)
-            fsg_build_fe_bla(r->dev, Mbla, rbla, R.bla_len, bla_f, R.bla_nit, bla_first,
-                             bla_first_step, kc, bla_chain, bla_chain_step, s);
+            fsg_build_fe_bla(r->dev, Mbla, rbla, R.bla_len, bla_f, R.bla_nit, bla_at, kc, s);
         else if (R.flavor != 0)
             fsg_build_bs_fr_bla(Mbs, rbla, R.bla_len, bs_blaf, bs_rf, s);
     }

@@ -50,13 +50,15 @@ struct RefDev {
                                 // (rounded down with a 2^-20 margin), r exponent,
                                 // A exponent, B exponent},
                                 // [2i + 1] = {A.x, A.y, B.x, B.y} float bits
-    const int4 *bla_first;      // [2 bla_nit] per start index it = w / 8, the first
-                                // stage ref_BLA_get tries there: its bla_f record
-    const int *bla_first_step;  // [bla_nit] that stage's step, 0 when none is tried
-    const int4 *bla_chain;      // [2 bla_nit] per start index, the composite of the run of
-                                // first candidates from there (header and payload as bla_f)
-    const int2 *bla_chain_step; // [bla_nit] {iterations of that run, its BLA steps}, {0, 0}
-                                // when none is stored
+    const int4 *bla_at;         // [5 bla_nit] per start index it = w / 8: the first stage
+                                // ref_BLA_get tries there and the composite of the run of
+                                // first candidates from there (fsg_ref.cu):
+                                // {f mantissa^2 bits, 2 f exponent, c mantissa^2 bits,
+                                // 2 c exponent} of the radii f of the first stage (sign
+                                // bit: no smaller stage either when it is refused) and c
+                                // of the run (0: none stored), then of the first stage
+                                // {A exponent, B exponent, step, 0}, {A.x, A.y, B.x, B.y}
+                                // and of the run the same
     int bla_nit;                // (len >> 3) + 1
     const int4 *fe_runs;        // [5 (len + 1)] per position w, the composed map of the
                                 // fast steps from w to the next multiple of 8 (fsg_ref.cu,

@@ -187,34 +187,51 @@ __device__ __forceinline__ bool bla_ok(const Lane &s, int4 H) {
     return fmaf(s.ux, s.ux, s.uy * s.uy) < (rm * rm) * __int_as_float((d + 127) << 23);
 }
 
+// bla_ok against the squared radius of a bla_at record (its sign is a flag);
+// m2 = |u|^2
+__device__ __forceinline__ bool at_ok(float m2, int E, int r2, int re2) {
+    const int d = min(max(re2 - 2 * E, -126), 126);
+    return m2 < fabsf(__int_as_float(r2)) * __int_as_float((d + 127) << 23);
+}
+
 // ref_BLA_get (perturbation.py:2116-2170): the largest stage from
 // 3 + ctz(w >> 3) (capped at stages - 1) down to 3 whose step is below
 // first_invalid - w and whose radius admits dz.  The first candidate of each
-// start index (header, payload and step) is tabulated when the reference is
-// built.  Radii of one start index never grow with the stage (a parent's r is
+// start index is tabulated when the reference is built, with the run of first
+// candidates from there, composed, which is taken where its radius admits dz: it
+// is at most 0.9 of the first candidate's, a margin above the FP32 test's
+// rounding.  Radii of one start index never grow with the stage (a parent's r is
 // min(r of its first child, ...), :2023-2024), so when stage 3 refuses, every
 // stage does: after the first candidate the search tests stage 3, then the
-// stages between.
-__device__ __forceinline__ int bla_find(const int4 *__restrict__ T, const int4 *__restrict__ FF,
-                                        const int *__restrict__ FS, const Lane &s, int w,
-                                        int4 &H, int4 &P) {
+// stages between.  Returns the step, H = {A exponent, B exponent, ...}, P.
+__device__ __forceinline__ int bla_find(const int4 *__restrict__ T, const int4 *__restrict__ AT,
+                                        const Lane &s, int w, int4 &H, int4 &P) {
     const int it = w >> FSG_STG_COMPRESSED;
-    const int st = __ldg(&FS[it]);
-    H = __ldg(&FF[2 * it]);
-    P = __ldg(&FF[2 * it + 1]);
-    if (st == 0) return 0;
-    const int i0 = 2 * it;
+    const int4 *at = AT + 5 * it;
+    const int4 r = __ldg(at);
+    const float m2 = fmaf(s.ux, s.ux, s.uy * s.uy);
+    if (at_ok(m2, s.E, r.x, r.y)) {
+        at += at_ok(m2, s.E, r.z, r.w) ? 3 : 1;
+        H = __ldg(at);
+        P = __ldg(at + 1);
+        return H.z;
+    }
+    if (r.x < 0) return 0;
+    const int i0 = 2 * it, st = __ldg(at + 1).z;
     // BLA_index(i, stg) = 2 i + 2^stg - 1 over the stored stages (stg - 3)
-    if (bla_ok(s, H)) return st;
-    if (st == 8) return 0;
     const int4 H3 = __ldg(&T[2 * i0]);
     if (!bla_ok(s, H3)) return 0;
     for (int stg = 30 - __clz(st); stg > FSG_STG_COMPRESSED; stg--) {
         const int idx = i0 + (1 << (stg - FSG_STG_COMPRESSED)) - 1;
-        H = __ldg(&T[2 * idx]);
-        if (bla_ok(s, H)) { P = __ldg(&T[2 * idx + 1]); return 1 << stg; }
+        const int4 h = __ldg(&T[2 * idx]);
+        if (bla_ok(s, h)) {
+            H.x = h.z; H.y = h.w;
+            P = __ldg(&T[2 * idx + 1]);
+            return 1 << stg;
+        }
     }
-    H = H3; P = __ldg(&T[2 * i0 + 1]);
+    H.x = H3.z; H.y = H3.w;
+    P = __ldg(&T[2 * i0 + 1]);
     return 1 << FSG_STG_COMPRESSED;
 }
 
@@ -261,18 +278,15 @@ __device__ __forceinline__ int pixel_fe32(const TileDev &T, const CalcDev &C, lo
     te -= 1;
     const int xrsem = C.xrsem, max_iter = C.max_iter;
     const int order = R.order, div_iter = R.div_iter, first_invalid = R.first_invalid;
-    const bool bla_on = C.bla && R.bla_first != nullptr;
+    const bool bla_on = C.bla && R.bla_at != nullptr;
     // escape test on the table's 2 Z: |2 Z|^2 > 4 M^2
     const float M2f = (float)C.M2, M2f4 = 4.f * M2f;
     const int4 *__restrict__ Zp = R.Zp;
     const int4 *__restrict__ dZndc_f = R.dZndc_f;
     const int4 *__restrict__ dZndz_f = R.dZndz_f;
     const int4 *__restrict__ bla_f = R.bla_f;
-    const int4 *__restrict__ bla_first = R.bla_first;
-    const int *__restrict__ bla_first_step = R.bla_first_step;
+    const int4 *__restrict__ bla_at = R.bla_at;
     const int4 *__restrict__ fe_runs = R.fe_runs;
-    const int4 *__restrict__ bla_chain = R.bla_chain;
-    const int2 *__restrict__ bla_chain_step = R.bla_chain_step;
     // c from the pixel (perturbation.py:2214-2230) in Xrange, then fe
     double2 pp = fsg_pixel(T, ip);
     double x1 = T.lin[0] * pp.x + T.lin[1] * pp.y;
@@ -299,28 +313,14 @@ __device__ __forceinline__ int pixel_fe32(const TileDev &T, const CalcDev &C, lo
         // continue saw w < div_iter - 1, or a BLA jump stopped short of it)
         if (bla_on && (w & 7) == 0 && w < first_invalid) {
             int4 H, P;
-            int step = bla_find(bla_f, bla_first, bla_first_step, s, w, H, P);
-            // when the first candidate is taken, the run of first candidates
-            // from here, composed (its radius is at most 0.9 of the first
-            // candidate's: the margin covers the FP32 test's rounding)
-            if (step != 0 && step == __ldg(&bla_first_step[w >> FSG_STG_COMPRESSED])) {
-                const int2 cs = __ldg(&bla_chain_step[w >> FSG_STG_COMPRESSED]);
-                if (cs.y >= 2) {
-                    const int4 Hc = __ldg(&bla_chain[2 * (w >> FSG_STG_COMPRESSED)]);
-                    if (bla_ok(s, Hc)) {
-                        H = Hc;
-                        P = __ldg(&bla_chain[2 * (w >> FSG_STG_COMPRESSED) + 1]);
-                        step = cs.x;
-                    }
-                }
-            }
+            const int step = bla_find(bla_f, bla_at, s, w, H, P);
             if (step != 0) {
                 const float Ax = __int_as_float(P.x), Ay = __int_as_float(P.y);
                 const float Bx = __int_as_float(P.z), By = __int_as_float(P.w);
                 // dz' = A dz + B dc on the exponent En = max(E + Ae, Ec + Be - 60,
                 // Ec - 100): A dz scaled by 2^(E + Ae - En) <= 1, B dc by
                 // 2^(Ec + Be - En) <= 2^60 (terms below 2^-127 of the scale vanish)
-                const int Ea = s.E + H.z, Eb = Ec + H.w;
+                const int Ea = s.E + H.x, Eb = Ec + H.y;
                 const int En = max(max(Ea, Eb - 60), Ec - 100);
                 const float sa = __int_as_float((max(Ea - En, -127) + 127) << 23);
                 const float sb = __int_as_float((max(Eb - En, -127) + 127) << 23);
@@ -331,12 +331,12 @@ __device__ __forceinline__ int pixel_fe32(const TileDev &T, const CalcDev &C, lo
                 if ((unsigned)(mag_b(s) - 97) > 60u) renorm_u(s, cmx, cmy, Ec);
                 if (dzndc_on) {
                     float vx = Ax * s.vx - Ay * s.vy, vy = Ax * s.vy + Ay * s.vx;
-                    s.vx = vx; s.vy = vy; s.F += H.z;
+                    s.vx = vx; s.vy = vy; s.F += H.x;
                     renorm_v(s.vx, s.vy, s.F);
                 }
                 if (dzndz_on) {
                     float qx = Ax * s.qx - Ay * s.qy, qy = Ax * s.qy + Ay * s.qx;
-                    s.qx = qx; s.qy = qy; s.G += H.z;
+                    s.qx = qx; s.qy = qy; s.G += H.x;
                     renorm_v(s.qx, s.qy, s.G);
                 }
                 n += step;

@@ -774,18 +774,22 @@ __global__ void k_fe_bla(const double2 *M, const double *r, int n, int4 *F) {
 
 // the first stage ref_BLA_get (perturbation.py:2116-2170) tries at each start
 // index it = w / 8: 3 + ctz(it) capped at stages - 1 (stages - 1 for it = 0),
-// lowered to the largest stage whose step is below first_invalid - w; its
-// bla_f record is copied beside it so that the kernel's first test needs one
-// load.  Where stage 3 has radius 0 no stage of the index admits any dz
-// (radii never grow with the stage, :2023-2024; 0 < r is strict): step 0, no
-// lookup -- at the orbit's critical point Z_0 = 0 (A = 2 Z_0 = 0, r = 0) the
-// search failed once per period
-__global__ void k_fe_bla_first(const RefDev *Rp, const int4 *F, int nit, int4 *FF, int *FS) {
+// lowered to the largest stage whose step is below first_invalid - w.  Where
+// stage 3 has radius 0 no stage of the index admits any dz (radii never grow
+// with the stage, :2023-2024; 0 < r is strict): radius and step 0 -- at the
+// orbit's critical point Z_0 = 0 (A = 2 Z_0 = 0, r = 0) the search failed once
+// per period.  The sign of the squared mantissa tells the kernel that nothing is
+// left to try when this stage is refused (step 0 or 8).  Everything a lookup
+// reads stands in one record, the two radii in its first word: a declined
+// attempt is one load, a taken one three (a table each for steps, radii and
+// payloads of the first stage and of the run took six).
+__device__ __forceinline__ int sq_bits(float m) { return __float_as_int(m * m); }
+__global__ void k_fe_bla_first(const RefDev *Rp, const int4 *F, int nit, int4 *AT) {
     const RefDev &R = *Rp;
     int it = blockIdx.x * blockDim.x + threadIdx.x;
     if (it >= nit) return;
     const int inv = R.first_invalid - (it << 3);
-    int4 h = make_int4(0, FE_ZERO_E, 0, 0), p = make_int4(0, 0, 0, 0);
+    int4 h = make_int4(0, 0, 0, 0), p = make_int4(0, 0, 0, 0);
     int step = 0;
     if (inv > 8 && R.stages - 1 >= 3) {
         int top = R.stages - 1;
@@ -796,7 +800,12 @@ __global__ void k_fe_bla_first(const RefDev *Rp, const int4 *F, int nit, int4 *F
             if (idx < R.bla_len) { h = F[2 * idx]; p = F[2 * idx + 1]; step = 1 << top; }
         }
     }
-    FF[2 * it] = h; FF[2 * it + 1] = p; FS[it] = step;
+    int4 *o = AT + 5 * (size_t)it;
+    // (radius 0: no exponent)
+    o[0] = make_int4(sq_bits(__int_as_float(h.x)) | (step <= 8 ? (int)0x80000000 : 0),
+                     h.x != 0 ? 2 * h.y : 0, 0, 0);
+    o[1] = make_int4(h.z, h.w, step, 0);
+    o[2] = p;
 }
 
 // |a| of an Xrange complex as a double (0 below, inf above the double range)
@@ -818,8 +827,7 @@ __device__ __forceinline__ double xabs_d(xc a) {
 // its number of steps.  A run stops before a step that would cut the radius
 // below a quarter of the shorter run's (a long run that rarely applies) and
 // after 64 steps; runs of fewer than 2 steps are not stored.
-__global__ void k_fe_bla_chain(const RefDev *Rp, const int *FS, int nit, double kc, int4 *CH,
-                               int2 *CS) {
+__global__ void k_fe_bla_chain(const RefDev *Rp, int nit, double kc, int4 *AT) {
     const RefDev &R = *Rp;
     const int it = blockIdx.x * blockDim.x + threadIdx.x;
     if (it >= nit) return;
@@ -827,7 +835,7 @@ __global__ void k_fe_bla_chain(const RefDev *Rp, const int *FS, int nit, double 
     double rc = -1.;                       // < 0: no bound yet
     int j = it, total = 0, count = 0;
     while (j < nit && count < 64) {
-        const int step = FS[j];
+        const int step = AT[5 * (size_t)j + 1].z;
         if (step == 0) break;
         const int idx = 2 * j + (step >> FSG_STG_COMPRESSED) - 1;
         if (idx >= R.bla_len) break;
@@ -844,22 +852,20 @@ __global__ void k_fe_bla_chain(const RefDev *Rp, const int *FS, int nit, double 
         total += step; count++;
         j += step >> FSG_STG_COMPRESSED;
     }
-    int4 h = make_int4(0, FE_ZERO_E, 0, 0), p = make_int4(0, 0, 0, 0);
+    int4 h = make_int4(0, 0, 0, 0), p = make_int4(0, 0, 0, 0);
     if (count >= 2 && rc > 0. && rc < INFINITY) {
         const fe a = fe_norm(fe_from_xc(P)), b = fe_norm(fe_from_xc(Q));
         const fe rf = fe_norm(fe_from_d(cx(0.9 * rc, 0.)));
         if (rf.e != FE_ZERO_E && a.e != FE_ZERO_E) {
-            h = make_int4(__float_as_int(rf.x), rf.e, a.e, b.e);
+            h = make_int4(sq_bits(rf.x), 2 * rf.e, a.e, b.e);
             p = make_int4(__float_as_int(a.x), __float_as_int(a.y), __float_as_int(b.x),
                           __float_as_int(b.y));
-        } else {
-            total = 0; count = 0;
         }
-    } else {
-        total = 0; count = 0;
     }
-    CH[2 * it] = h; CH[2 * it + 1] = p;
-    CS[it] = make_int2(total, count);
+    int4 *o = AT + 5 * (size_t)it;
+    ((int2 *)o)[1] = make_int2(h.x, h.y);
+    o[3] = make_int4(h.z, h.w, total, 0);
+    o[4] = p;
 }
 
 // ---------------------------------------------------------------------------
@@ -1111,15 +1117,11 @@ void fsg_build_fe_paths(int len, const double2 *dzndc, const double2 *dzndc_xm,
 }
 
 void fsg_build_fe_bla(const RefDev *Rd, const double2 *Mbla, const double *rbla, int bla_len,
-                      int4 *bla_f, int bla_nit, int4 *bla_first, int *bla_first_step,
-                      double kc, int4 *bla_chain, int2 *bla_chain_step, cudaStream_t s) {
+                      int4 *bla_f, int bla_nit, int4 *bla_at, double kc, cudaStream_t s) {
     int tb = 256;
     if (bla_f && bla_len > 0) {
         k_fe_bla<<<(bla_len + tb - 1) / tb, tb, 0, s>>>(Mbla, rbla, bla_len, bla_f);
-        k_fe_bla_first<<<(bla_nit + tb - 1) / tb, tb, 0, s>>>(Rd, bla_f, bla_nit, bla_first,
-                                                              bla_first_step);
-        if (bla_chain)
-            k_fe_bla_chain<<<(bla_nit + tb - 1) / tb, tb, 0, s>>>(Rd, bla_first_step, bla_nit, kc,
-                                                                  bla_chain, bla_chain_step);
+        k_fe_bla_first<<<(bla_nit + tb - 1) / tb, tb, 0, s>>>(Rd, bla_f, bla_nit, bla_at);
+        k_fe_bla_chain<<<(bla_nit + tb - 1) / tb, tb, 0, s>>>(Rd, bla_nit, kc, bla_at);
     }
 }
