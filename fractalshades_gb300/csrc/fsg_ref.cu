@@ -697,7 +697,8 @@ __global__ void k_fe_runs(const RefDev *Rp, const int4 *Zp, const int4 *Df, int 
     if (w > len) return;
     int4 *o = out + 5 * (size_t)w;
     const int k = 8 - (w & 7);
-    bool ok = k >= 2 && w + k <= len;
+    // (inside the orbit, its period, and ahead of the reference's divergence)
+    bool ok = k >= 2 && w + k <= min(len, Rp->order) && w + k <= Rp->div_iter - 1;
     double2 P = cx(odd ? 0. : 1., 0.), Rm = cx(0., 0.);      // (Q and S in the odd lane)
     int eR = 0;
     double amax = 0., z2max = 0.;

@@ -121,3 +121,29 @@ def test_claim_order_of_rectangles(ctx, mode, nx, ny):
     assert (a[1] > 0).all()
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("M", [4., 30., 1e3, 1e8, 1e17])
+def test_fe32_escape_radius(ctx, M):
+    """The FP32 loop leaves the escape test out where the orbit's exponent
+    rules an escape out; from the values at a radius of 2.5, plain iteration
+    tells at which step a larger one is passed."""
+    w = syn.seahorse_workload(nx=40, max_iter=6000)
+    ref = _reference(ctx, w, False)
+    w.M = 2.5
+    Z0, si0, sr0 = _run(ctx, w, ref, "fe32")
+    w.M = M
+    Z, si, sr = _run(ctx, w, ref, "fe32")
+    assert (sr0 == 1).all() and (sr == 1).all()
+    dx = float(np.ldexp(w.dx_m, w.dx_e))
+    c = complex(w.center) + dx * (w.xs[None, :] + 1j * w.ys[:, None]).ravel()
+    z, more = Z0[0].copy(), np.zeros(Z0.shape[1], dtype=np.int64)
+    for _ in range(12):
+        go = np.abs(z) <= M
+        z = np.where(go, z * z + c, z)
+        more += go
+    # the FP32 values are good to about 1e-4 of |z| here and double that at each
+    # further step; a pixel that lands on the radius to within that may take one
+    # step more or less, which a few steps of squaring make rare
+    off = si[0] - si0[0] != more
+    assert off.sum() <= 0.01 * off.size and np.abs(si[0] - si0[0] - more).max() <= 1
