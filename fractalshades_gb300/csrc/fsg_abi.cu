@@ -41,8 +41,8 @@ void fsg_build_fe_paths(int len, const double2 *dzndc, const double2 *dzndc_xm,
 void fsg_build_fe_bla(const RefDev *Rd, const double2 *Mbla, const double *rbla, int bla_len,
                       int4 *bla_f, int bla_nit, int4 *bla_at, double kc, cudaStream_t s);
 void fsg_build_bs_fr(const RefDev *Rd, int len, int4 *Zf, const double *dXa, const double *dXb,
-                     const double *dYa, const double *dYb, int4 *hf, float4 *fa, int4 *fz,
-                     float4 *fh, int div_iter, cudaStream_t s);
+                     const double *dYa, const double *dYb, int4 *hf, int4 *at, int div_iter,
+                     cudaStream_t s);
 void fsg_build_bs_fr_bla(const double *Mbs, const double *rbla, int bla_len, int4 *blaf,
                          int2 *rf, cudaStream_t s);
 
@@ -1023,23 +1023,18 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
     // FP32+exp tables (Burning Ship)
     int4 *bs_Zf = nullptr, *bs_hf = nullptr, *bs_blaf = nullptr;
     int2 *bs_rf = nullptr;
-    float4 *bs_fa = nullptr, *bs_fh = nullptr;
-    int4 *bs_fz = nullptr;
+    int4 *bs_at = nullptr;
     if (d->flavor != 0) {
         RA(bs_Zf, len + 1);
-        RA(bs_fa, len + 1);
-        RA(bs_fz, len + 1);
-        if (d->calc_dzndc) {
-            RA(bs_hf, 2 * (size_t)(len + 1));
-            RA(bs_fh, len + 1);
-        }
+        RA(bs_at, 3 * (size_t)(len + 1));
+        if (d->calc_dzndc) RA(bs_hf, 2 * (size_t)(len + 1));
         if (R.bla_len > 0) {
             RA(bs_blaf, 4 * (size_t)R.bla_len);
             RA(bs_rf, (size_t)R.bla_len);
         }
     }
     R.bs_Zf = bs_Zf; R.bs_hf = bs_hf; R.bs_blaf = bs_blaf; R.bs_rf = bs_rf;
-    R.bs_fa = bs_fa; R.bs_fz = bs_fz; R.bs_fh = bs_fh;
+    R.bs_at = bs_at;
     RCK(ref_malloc(ctx, (void **)&r->dev, sizeof(RefDev)), "cudaMallocAsync(reference descriptor)");
     RCK(cudaMemcpyAsync(r->dev, &R, sizeof(RefDev), cudaMemcpyHostToDevice, s), "upload descriptor");
     // Builds.  The derivative paths are serial walks of one block; what needs
@@ -1077,7 +1072,7 @@ int fsg_ref_create(fsg_ctx *ctx, const fsg_ref_desc *d, fsg_ref **out) {
             RCK(cudaStreamSynchronize(side), "reference table build");
     }
     if (d->flavor != 0)
-        fsg_build_bs_fr(r->dev, len, bs_Zf, dXa, dXb, dYa, dYb, bs_hf, bs_fa, bs_fz, bs_fh,
+        fsg_build_bs_fr(r->dev, len, bs_Zf, dXa, dXb, dYa, dYb, bs_hf, bs_at,
                         R.div_iter, s);
     if (fe_tables) {
         fsg_build_fe_paths(len, dzndc, dzndc_xm, dzndc_xe, dzndc_f, dzndz, dzndz_xm, dzndz_xe,

@@ -948,10 +948,8 @@ template <> struct IsXr<xf> { static constexpr bool value = true; };
 // FL: the flavor as a compile-time constant (1..5), or 0 to read C.flavor.  AXIS:
 // every reference of the launch is real (RefDev.axis), flavor 1
 template <class T, int FL, bool AXIS>
-FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
-                      unsigned long long &full_, unsigned long long &bla_,
-                      unsigned long long &reb_, unsigned long long &itsum) {
-    unsigned nfull = 0, nbla = 0, nreb = 0;
+FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned &nfull,
+                     unsigned &nbla, unsigned &nreb) {
     const TileDev &Tl = T_;
     const RefDev &R = *Tl.ref;
     const long long np = (long long)Tl.nx * Tl.ny;
@@ -1019,9 +1017,23 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
             // (0), a BLA step was taken (1), the step at w has to run in fr (2) or
             // the tests at w have to (3); the fr values are current on return.
             auto frame_run = [&]() -> int {
-                int4 fz = __ldg(&R.bs_fz[w]);
+                // the records of w, read together as soon as w is known
+                int4 fz;
+                float4 fa, Hm = make_float4(0.f, 0.f, 0.f, 0.f);
+                auto fetch = [&]() {
+                    const int4 *at = R.bs_at + 3 * (size_t)w;
+                    fz = __ldg(at);
+                    fa = __ldg((const float4 *)at + 1);
+                    if (hess) Hm = __ldg((const float4 *)at + 2);
+                };
+                fetch();
+                const bool bla_on = C.bla && R.bla_len > 0;
+                // X_0 = Y_0 = 0 and no BLA attempt there: after a rebase the step
+                // at w = 0 follows at once
+                const bool crit0 = FL == 1 && (__ldg(&R.bs_at[0]).x & 4)
+                                   && !(bla_on && (1 << FSG_STG_COMPRESSED) < R.first_invalid);
                 for (;;) {
-                    if (C.bla && R.bla_len > 0 && (w & 7) == 0 &&
+                    if (bla_on && (w & 7) == 0 &&
                         (1 << FSG_STG_COMPRESSED) < R.first_invalid - w && bla_possible(R, w)) {
                         int ib;
                         const int step = BLAGet<T>::get(R, fr_norm(Fm.ux, Fm.E),
@@ -1033,17 +1045,13 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
                         }
                     }
                     if (!(fz.x & 5)) { frame_out(Fm, xn, yn, h); return 2; }
-                    float4 Hm = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (hess && !dyn) Hm = __ldg(&R.bs_fh[w]);
                     if (fz.x & 4) {
                         if (FL == 1 && dyn) bs_frame_zero1(hess, Fm);
                         else bs_frame_step_zero(flavor, hess, Fm, Hm, fz.y, dyn);
                     } else if (AXIS) {
-                        const float4 fa = __ldg(&R.bs_fa[w]);
                         if (Fm.s == 0.f) bs_frame_step_axis1<true>(hess, Fm, fa.x, fa.y, Hm, fz.y, dyn);
                         else bs_frame_step_axis1<false>(hess, Fm, fa.x, fa.y, Hm, fz.y, dyn);
                     } else {
-                        const float4 fa = __ldg(&R.bs_fa[w]);
                         const int eX = __float_as_int(fa.z), eY = __float_as_int(fa.w);
                         const bool ok = Fm.s == 0.f
                             ? bs_frame_step<true>(flavor, hess, Fm, fa.x, fa.y, eX, eY, Hm,
@@ -1055,31 +1063,42 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
                             return 2;
                         }
                     }
+                after_step:
+                    w += 1;
+                    if (w >= order) w = 0;                  // w < order before
+                    fetch();
                     frame_renorm(Fm);
                     n += 1;
                     nfull++;
-                    if (n >= C.max_iter) { stop = 0; frame_out(Fm, xn, yn, h); return 0; }
-                    w += 1;
-                    if (w >= order) w = w % order;
-                    fz = __ldg(&R.bs_fz[w]);
+                    if (n >= C.max_iter) {
+                        // (the step that reaches it leaves w where it was)
+                        w = (w == 0 ? order : w) - 1;
+                        stop = 0; frame_out(Fm, xn, yn, h); return 0;
+                    }
                     // deltas below the orbit point's bound: no escape, no rebase
                     const int ed = Fm.E + fr_fexp(fmaxf(fabsf(Fm.ux), fabsf(Fm.uy)));
                     if (ed <= min(fz.z, eMlim) && fz.w <= eMlim) { dyn = false; continue; }
                     const bool divr = w >= div_iter - 1;
                     int res = 3;
-                    if (fz.x & 2) {
-                        const float4 fb = __ldg(&R.bs_fa[w]);
-                        res = bs_frame_tests(Fm, fb.x, fb.y, __float_as_int(fb.z),
-                                             AXIS ? FR_ZERO_E : __float_as_int(fb.w), M2s, divr);
+                    if ((fz.x & 4) && ed <= eMlim && Fm.E <= 10) {
+                        res = 2;               // X = Y = 0, no escape
+                    } else if (fz.x & 2) {
+                        res = bs_frame_tests(Fm, fa.x, fa.y, __float_as_int(fa.z),
+                                             AXIS ? FR_ZERO_E : __float_as_int(fa.w), M2s, divr);
                     }
                     if (res == 0) { dyn = false; continue; }
                     if (res == 1) { stop = 1; frame_out(Fm, xn, yn, h); return 0; }
                     if (res == 2) {
                         // rebase where X + xn, Y + yn round to the deltas: they stay
-                        if (hess) frame_add_hess(Fm, __ldg(&R.bs_fh[w]), fz.y);
+                        if (hess) frame_add_hess(Fm, Hm, fz.y);
                         if (!divr) dyn = true;
+                        const bool there = w == 0;
                         w = 0; nreb++;
-                        fz = __ldg(&R.bs_fz[0]);
+                        if (FL == 1 && dyn && crit0) {
+                            bs_frame_zero1(hess, Fm);
+                            goto after_step;
+                        }
+                        if (!there) fetch();
                         continue;
                     }
                     frame_out(Fm, xn, yn, h);
@@ -1123,7 +1142,7 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
             }
             if (n >= C.max_iter) { stop = 0; break; }
             w += 1;
-            if (w >= order) w = w % order;
+            if (w >= order) w = 0;
         }
         if constexpr (XR_FORM) {
             // the Xrange branch's tests (perturbation.py:1627-1731): escape on
@@ -1208,7 +1227,7 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
         if constexpr (FR_FORM) {
             // the frame form takes over while the deltas stay below 2^11 and
             // the next step can run there
-            if (max(xn.e, yn.e) <= 10 && (__ldg(&R.bs_fz[w]).x & 5)) {
+            if (max(xn.e, yn.e) <= 10 && (__ldg(&R.bs_at[3 * (size_t)w]).x & 5)) {
                 frame_in(Fm, xn, yn, h);
                 frm = true;
             }
@@ -1259,26 +1278,38 @@ FSG_DEV void pixel_bs(const TileDev &T_, const CalcDev &C, long long ip,
     Tl.stop_iter[ip] = n; Tl.stop_reason[ip] = stop;
     double absd = 0.5 * (hypot(hd[0] + hd[3], hd[1] - hd[2]) + hypot(hd[0] - hd[3], hd[1] + hd[2]));
     fsg_epilogue(Tl, C, ip, cx(xo, yo), absd, n);
-    itsum += (unsigned long long)n;
-    full_ += nfull; bla_ += nbla; reb_ += nreb;
+    return n;
 }
 
-// the FP32 + exponent kernels hold three 256-thread blocks per SM (at most 85
-// registers a thread), the others two (128): flavor 1 in the double form, 255^2
-// pixels of the period-12 nucleus to 20000 iterations, takes 68 ms with them, 95
-// ms at its own 156 registers and one block, 73 ms at 80 with spills
+// The FP32 + exponent kernels hold four 256-thread blocks per SM (at most 64
+// registers a thread: short chains of FP32 and integer operations want warps more
+// than registers -- flavor 1, 640^2 pixels of a period-3 nucleus to 20000
+// iterations, takes 45.5 ms so, 48.0 with three blocks, 48.9 with five, 60.6 with
+// two), flavor 5 three (its views spend more in the fr steps, which spill: 31 to 34
+// ms, 35 with four); the others two (128): flavor 1 in the double form, 255^2 pixels
+// of the period-12 nucleus to 20000 iterations, takes 67 ms with them, 95 ms at
+// its own 156 registers and one block, 73 ms at 80 with spills
 template <class T, int FL, bool AXIS>
-__global__ void __launch_bounds__(256, IsFr<T>::value ? 3 : 2)
+__global__ void __launch_bounds__(256, IsFr<T>::value ? (FL == 5 ? 3 : 4) : 2)
 k_perturb_bs(WorkDev W, CalcDev C) {
-    extern __shared__ long long s_start[];          // [W.ntiles + 1], sized at launch
+    // sized at launch: per-thread statistics (64-bit sums would hold 8 registers
+    // in the loop), then the pixel offsets of the launch's tiles
+    extern __shared__ unsigned long long bs_smem[];
+    unsigned long long *acc = bs_smem + threadIdx.x;           // acc[k * blockDim.x]
+    long long *s_start = (long long *)(bs_smem + 4 * blockDim.x);
+    const int nb = blockDim.x;
+    for (int k = 0; k < 4; k++) acc[k * nb] = 0ULL;
     fsg_load_starts(W, s_start);
-    unsigned long long nfull = 0, nbla = 0, nreb = 0, itsum = 0;
     int t; long long ip;
     while (true) {
         if (!fsg_claim_poll(W, s_start, t, ip)) break;
-        const unsigned long long before = itsum;
-        pixel_bs<T, FL, AXIS>(W.tiles[t], C, ip, nfull, nbla, nreb, itsum);
-        fsg_account(W, itsum - before);
+        unsigned nfull = 0, nbla = 0, nreb = 0;
+        const int n = pixel_bs<T, FL, AXIS>(W.tiles[t], C, ip, nfull, nbla, nreb);
+        fsg_account(W, (unsigned long long)n);
+        acc[0] += (unsigned long long)n;
+        acc[nb] += nfull;
+        acc[2 * nb] += nbla;
+        acc[3 * nb] += nreb;
     }
-    fsg_flush_stats(W, itsum, nfull, nbla, nreb);
+    fsg_flush_stats(W, acc[0], acc[nb], acc[2 * nb], acc[3 * nb]);
 }

@@ -7,7 +7,7 @@
 
 template <int FL, bool AXIS>
 static void launch_bs_fr(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s) {
-    const size_t sm = fsg_starts_smem(W);
+    const size_t sm = fsg_starts_smem(W) + 4 * sizeof(unsigned long long) * (size_t)block;
     k_perturb_bs<fr, FL, AXIS><<<fsg_auto_grid(k_perturb_bs<fr, FL, AXIS>, grid, block, W.total - W.base, sm),
                            block, sm, s>>>(W, C);
 }

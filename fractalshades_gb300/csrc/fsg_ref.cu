@@ -913,11 +913,11 @@ __global__ void k_bs_fr_bla(const double *M, const double *r, int n, int4 *out, 
     if (i < n) rf[i] = fr_pack(fr_from_d(r[i]));
 }
 
-// Frame-step tables (fsg_bs.cuh, BSFrame): per orbit index w
-//   fa[w] = {X, Y as floats, exponent of X, exponent of Y}: a component of
+// Frame-step records (fsg_bs.cuh, BSFrame): per orbit index w
+//   at[3 w + 1] = {X, Y as floats, exponent of X, exponent of Y}: a component of
 //           magnitude in [2^-60, 2^40) is its float value; one below 2^-100 is
 //           a signed zero (its exponent stays exact); 0 has FR_ZERO_E
-//   fz[w] = {flags, g, Tw, eZ}: flags bit 0, the frame step may run at w (one
+//   at[3 w] = {flags, g, Tw, eZ}: flags bit 0, the frame step may run at w (one
 //           component in [2^-60, 2^40), the other 0, below 2^-100 or in that
 //           range); bit 1, the loop's tests can run at w (each component 0,
 //           below 2^-100 or in [2^-60, 2^40)); bit 2, X = Y = 0 (the step
@@ -928,7 +928,7 @@ __global__ void k_bs_fr_bla(const double *M, const double *r, int n, int4 *out, 
 //           (FR_ZERO_E where the tests must run: X = Y = 0, a component
 //           outside the float range, w >= div_iter - 1); eZ the exponent of
 //           max(|X|, |Y|)
-//   fh[w] = {dXa, dXb, dYa, dYb} * 2^-g, entries below 2^-126 of the
+//   at[3 w + 2] = {dXa, dXb, dYa, dYb} * 2^-g as floats, entries below 2^-126 of the
 //           largest read as 0
 __device__ __forceinline__ int fr_frame_kind(fr v) {    // 0 zero, 1 tiny, 2 float, 3 other
     if (v.m == 0.f) return 0;
@@ -945,8 +945,7 @@ __device__ __forceinline__ float fr_rel(fr v, int g) {
     const int k = v.e - g;
     return k < -126 ? 0.f : v.m * __int_as_float((k + 127) << 23);
 }
-__global__ void k_bs_frame_tab(const int4 *Zf, const int4 *hf, int n, int div_iter, float4 *fa,
-                               int4 *fz, float4 *fh) {
+__global__ void k_bs_frame_tab(const int4 *Zf, const int4 *hf, int n, int div_iter, int4 *at) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 z = Zf[i];
@@ -957,6 +956,7 @@ __global__ void k_bs_frame_tab(const int4 *Zf, const int4 *hf, int n, int div_it
     if ((flags & 2) && (kx == 2 || ky == 2)) flags |= 1;
     if (kx == 0 && ky == 0) flags |= 4;
     int g = 0;
+    float4 *o = (float4 *)(at + 3 * (size_t)i), Hm = make_float4(0.f, 0.f, 0.f, 0.f);
     if (hf) {
         const int4 p = hf[2 * i], q = hf[2 * i + 1];
         fr h[4];
@@ -967,24 +967,25 @@ __global__ void k_bs_frame_tab(const int4 *Zf, const int4 *hf, int n, int div_it
         for (int k = 0; k < 4; k++)
             if (h[k].m != 0.f) { any = true; g = max(g, h[k].e); }
         if (!any) g = 0;
-        fh[i] = make_float4(fr_rel(h[0], g), fr_rel(h[1], g), fr_rel(h[2], g), fr_rel(h[3], g));
+        Hm = make_float4(fr_rel(h[0], g), fr_rel(h[1], g), fr_rel(h[2], g), fr_rel(h[3], g));
     }
-    fa[i] = make_float4(fr_frame_val(x, kx), fr_frame_val(y, ky), __int_as_float(x.e),
+    o[2] = Hm;
+    o[1] = make_float4(fr_frame_val(x, kx), fr_frame_val(y, ky), __int_as_float(x.e),
                         __int_as_float(y.e));
     int Tw = FR_ZERO_E, eZ = FR_ZERO_E;
     if (kx != 0) { Tw = max(Tw, x.e - 2); eZ = max(eZ, x.e); }
     if (ky != 0) { Tw = max(Tw, y.e - 2); eZ = max(eZ, y.e); }
     if (!(flags & 2) || i >= div_iter - 1) Tw = FR_ZERO_E;
-    fz[i] = make_int4(flags, g, Tw, eZ);
+    at[3 * (size_t)i] = make_int4(flags, g, Tw, eZ);
 }
 
 void fsg_build_bs_fr(const RefDev *Rd, int len, int4 *Zf, const double *dXa, const double *dXb,
-                     const double *dYa, const double *dYb, int4 *hf, float4 *fa, int4 *fz,
-                     float4 *fh, int div_iter, cudaStream_t s) {
+                     const double *dYa, const double *dYb, int4 *hf, int4 *at, int div_iter,
+                     cudaStream_t s) {
     int tb = 256;
     k_bs_fr_orbit<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Rd, Zf);
     if (hf) k_bs_fr_paths<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(dXa, dXb, dYa, dYb, len + 1, hf);
-    k_bs_frame_tab<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Zf, hf, len + 1, div_iter, fa, fz, fh);
+    k_bs_frame_tab<<<(len + 1 + tb - 1) / tb, tb, 0, s>>>(Zf, hf, len + 1, div_iter, at);
 }
 void fsg_build_bs_fr_bla(const double *Mbs, const double *rbla, int bla_len, int4 *blaf,
                          int2 *rf, cudaStream_t s) {
