@@ -938,6 +938,144 @@ FSG_DEV bool bs_step_ship(bool hess, double &xn, double &yn, double h[4], double
     return true;
 }
 
+// a1 b1 + a2 b2 (minus: a1 b1 - a2 b2): 58 binary orders apart only the larger
+// product is taken
+FSG_DEV double d_two_far(double a1, double b1, double a2, double b2, bool minus) {
+    const int e1 = d_field(a1) + d_field(b1), e2 = d_field(a2) + d_field(b2);
+    const unsigned flip = minus ? 0x80000000u : 0u;
+    if (abs(e1 - e2) >= 59 && max(e1, e2) >= 1025) {
+        const bool first = e1 > e2;
+        return d_mul_here(first ? a1 : d_flip(a2, flip), first ? b1 : b2);
+    }
+    return d_add_far(d_mul_here(a1, b1), d_flip(d_mul_here(a2, b2), flip));
+}
+
+// the exponent field of x, far below any for 0
+FSG_DEV int d_field0(double x) { return d_is0(x) ? -20000 : d_field(x); }
+// signs of products as words whose top bit counts
+FSG_DEV unsigned d_sgn2(double a, double b) { return d_hi(a) ^ d_hi(b); }
+FSG_DEV double d_zero_of(unsigned s) { return d_zero((s >> 31) != 0u); }
+
+// The same step at X = Y = +0 right after a rebase (the reference Hessian reads
+// as 0): products of deltas and c alone.  The plain form's other terms are zeros:
+// beside a sum that is not 0 they change nothing, and a sum of da or db that is 0
+// comes out as +0 whatever their signs (xa yn, xa 0 and yn 0 are not all negative).
+FSG_DEV bool bs_ship_crit(bool hess, double &xn, double &yn, double h[4], double a, double b) {
+    const int x = d_field(xn), y = d_field(yn);
+    if (max(x, y) > 1023 - 58 || min(x, y) == 0) return false;
+    // the fold's sign, its value only where it takes part in the sum with b
+    unsigned s1 = (d_hi(xn) ^ d_hi(yn)) & 0x80000000u;
+    double nx = a, ny = d_flip(b, 0x80000000u);
+    if (d_field(b) + 1023 - x - y < 59 || x + y < 1025) {
+        const double op = d_mul_here(xn, yn);
+        if (d_is0(op)) s1 = 0u;
+        ny = d_add_far(d_twice(d_flip(op, s1)), ny);
+    }
+    if (d_field(a) + 1023 - 2 * max(x, y) < 59) nx = d_add_far(d_two_far(xn, xn, yn, yn, true), a);
+    if (hess) {
+        const double xa = h[0], xb = h[1], ya = h[2], yb = h[3];
+        const int top = max(max(d_field0(xa), d_field0(xb)), max(d_field0(ya), d_field0(yb)));
+        if (top > 1900) return false;            // (infinities and NaN times a zero)
+        double da = 0., db = 0., na, nb;
+        if (max(x, y) + top <= 968) {
+            // every product underflows: the zeros' signs
+            na = d_zero_of(d_sgn2(xn, xa) & d_hi(xn) & ~(d_sgn2(yn, ya) & d_hi(yn)));
+            nb = d_zero_of(d_sgn2(xn, xb) & d_hi(xn) & ~(d_sgn2(yn, yb) & d_hi(yn)));
+        } else {
+            da = d_two_far(xa, yn, xn, ya, false);
+            db = d_two_far(xb, yn, xn, yb, false);
+            na = d_two_far(xn, xa, yn, ya, true);
+            nb = d_two_far(xn, xb, yn, yb, true);
+            if (d_is0(da)) da = 0.;
+            if (d_is0(db)) db = 0.;
+            if (d_is0(na) | d_is0(nb)) return false;
+        }
+        h[0] = d_twice(na);
+        h[1] = d_twice(nb);
+        h[2] = d_twice(d_flip(da, s1));
+        h[3] = d_twice(d_flip(db, s1));
+    }
+    xn = nx; yn = ny;
+    return true;
+}
+
+// bs_step_ship on the real axis far below the orbit (views whose deltas are 58
+// binary orders under X): products of two deltas are below half an ulp of the sum
+// that they enter, so neither they nor the sums are taken.  Exponent fields say
+// so for each sum (a product's exponent is the sum of its factors', or one more;
+// `far` binary orders leave a power of two its ulp): 10 products and 6 sums
+// remain of 18 and 15, which the FP64 pipe takes: a product there is one
+// instruction where the integer pipes take thirty, and the pipe is no longer what
+// bounds the loop (with two of the ten as integer products 8 % longer).  255^2
+// pixels of the period-12 nucleus to 20000 iterations: 67 ms without this step and
+// bs_ship_crit, 39 with them.  Yz, Xb, Ya: zeros, for the signs of results that are 0
+// because all their terms are.  false (nothing changed) where a sum is open.
+FSG_DEV bool bs_ship_deep(bool hess, double &xn, double &yn, double h[4], double X, double Yz, double Xa,
+                          double Xb, double Ya, double Yb, double a, double b) {
+    const int far = 55;
+    const int x = d_field(xn), y = d_field(yn), fX = d_field(X);
+    // (everything that the factors' fields can tell is settled ahead of the
+    // products: an integer test waits 100 clocks for an FP64 result)
+    bool ok = (fX - max(x, y) >= far + 3) & (min(x, y) >= 1) & (min(x, y) + fX >= 1025)
+              & (x + fX >= 2 * y + 2 + far);                 // yn yn beside xn (xn + 2 X)
+    const unsigned s1 = d_sgn2(yn, X) & 0x80000000u;
+    double n0 = 0., n1 = 0., n2 = 0., n3 = 0.;
+    if (hess) {
+        // exponents of da = ((xa yn + xn ya) + ya X) + yn Xa and of
+        // db = ((xb yn + xn yb) + xn Yb) + yb X
+        const double ha = h[0], hb = h[1], ga = h[2], gb = h[3];
+        const int xa = d_field0(ha), xb = d_field0(hb), ya = d_field0(ga), yb = d_field0(gb);
+        const int fXa = d_field(Xa), fYb = d_field(Yb);
+        const int sa = max(xa + y, x + ya) + 2, ta = ya + fX, ua = y + fXa;
+        const int sb = max(xb + y, x + yb) + 2, tb = x + fYb, ub = yb + fX;
+        const bool a3 = ya >= 1 && ta - sa >= far, b3 = tb - sb >= far;
+        ok &= (min(fXa, fYb) >= 1)
+              & (max(max(max(xa, xb), max(ya, yb)), max(max(fXa, fYb), fX)) <= 1900);
+        ok &= a3 | (ua - max(sa, ta + 2) >= far + 1);
+        ok &= b3 | ((yb >= 1) & (ub - max(sb, tb + 2) >= far + 1));
+        if (!ok) return false;
+        n2 = d_mul_here(yn, Xa);
+        n3 = d_mul_here(gb, X);
+        n0 = d_mul_here(Xa, xn);
+        n1 = d_mul_here(Yb, yn);                 // vb = yn yb + Yb yn
+        if (fYb - yb < far + 2) n1 = d_add_here(d_mul_here(yn, gb), n1);
+        n1 = d_flip(d_twice(n1), 0x80000000u);
+        if (a3) n2 = d_add_here(d_mul_here(ga, X), n2);
+        if (b3) n3 = d_add_here(d_mul_here(xn, Yb), n3);
+        n0 = d_add_here(d_mul_here(X, ha), n0);
+        n1 = d_add_here(d_twice(d_mul_here(X, hb)), n1);
+        // va = yn ya
+        if (!((d_field(n0) >= max(y + ya - 1023 + 2 + far, 1)) | (d_is0(n0) & (y + ya <= 968)))) return false;
+        n0 = d_twice(n0);
+        if (d_is0(n0) | d_is0(n1) | d_is0(n2) | d_is0(n3)) {
+            // with every term of the Hessian's steps underflowing: their signs
+            if (max(max(xa, xb), max(ya, yb)) + 1 + fX > 968 || max(ua, tb) > 968 || y + fYb > 968 || x + fXa > 968)
+                return false;
+            const unsigned pa = d_sgn2(ha, yn) & d_sgn2(xn, ga) & d_sgn2(ha, Yz) & d_sgn2(xn, Ya) & d_sgn2(ga, X) & d_sgn2(yn, Xa);
+            const unsigned pb = d_sgn2(hb, yn) & d_sgn2(xn, gb) & d_sgn2(hb, Yz) & d_sgn2(xn, Yb) & d_sgn2(gb, X) & d_sgn2(yn, Xb);
+            const unsigned da = d_sgn2(Xa, Yz) & d_sgn2(X, Ya), db = d_sgn2(X, Yb);
+            n0 = d_zero_of(d_sgn2(X, ha) & d_sgn2(Xa, xn) & ~(d_sgn2(yn, ga) & d_sgn2(Ya, yn)));
+            n1 = d_zero_of(d_sgn2(X, hb) & d_sgn2(Xb, xn) & ~(d_sgn2(yn, gb) & d_sgn2(Yb, yn)));
+            // ddiffabsdX (0 or -2) times the reference's d(XY), and ddiffabsdx times this
+            n2 = d_zero_of(s1 ? ~da & ~pa : da & pa);
+            n3 = s1 ? d_twice(d_mul_here(X, Yb)) : d_zero_of(db & pb);
+            h[0] = n0; h[1] = n1; h[2] = n2; h[3] = s1 ? d_twice(d_flip(n3, s1)) : n3;
+        } else {
+            if (s1) n3 = d_add_here(d_twice(d_mul_here(X, Yb)), n3);
+            if (min(min(d_field(n1), d_field(n2)), d_field(n3)) < 1) return false;
+            h[0] = n0; h[1] = n1; h[2] = d_twice(d_flip(n2, s1)); h[3] = d_twice(d_flip(n3, s1));
+        }
+    }
+    if (!ok) return false;
+    xn = d_add_here(d_mul_here(xn, d_twice(X)), a);
+    yn = d_add_here(d_twice(d_flip(d_mul_here(yn, X), s1)), d_flip(b, 0x80000000u));
+    return true;
+}
+
+// a + b; flavor 1 in the double form looks whether there is a sum to take
+template <class T, int FL> FSG_DEV T bs_add(T a, T b) { return a + b; }
+template <> FSG_DEV double bs_add<double, 1>(double a, double b) { return d_add_far(a, b); }
+
 template <class T> struct IsDouble { static constexpr bool value = false; };
 template <> struct IsDouble<double> { static constexpr bool value = true; };
 template <class T> struct IsFr { static constexpr bool value = false; };
@@ -975,6 +1113,11 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
     int w = 0, n = 0; signed char stop = -1; bool dyn = true;
     // double form: X_w + xn and Y_w + yn of the last test, while they stand
     double XX_last = 0., YY_last = 0.; bool has_sums = false;
+    // whether c is far enough below the orbit for bs_ship_crit and bs_ship_deep
+    bool below = false;
+    if constexpr (IsDouble<T>::value && FL == 1) {
+        below = max(d_field(a), d_field(b)) <= 1023 - 58;
+    }
     // calc_orbit snapshots (perturbation.py:1501-1508), the reference's two
     // forms only: the FP32 + exponent instantiation compiles without them
     constexpr bool FR_FORM = IsFr<T>::value;
@@ -1129,12 +1272,18 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
             if (hess && !dyn) BSRef<T>::hess(R, w, Xa, Xb, Ya, Yb);
             bool taken = false;
             if constexpr (IsDouble<T>::value && FL == 1) {
-                double xs = XX_last, ys = YY_last;
-                if (!has_sums) {
-                    xs = (d_is0(X) & !d_is0(xn)) ? xn : d_add_here(X, xn);
-                    ys = (d_is0(Y) & !d_is0(yn)) ? yn : d_add_here(Y, yn);
+                if (below) {
+                    if (dyn && (dbits(X) | dbits(Y)) == 0) taken = bs_ship_crit(hess, xn, yn, h, a, b);
+                    else if (AXIS) taken = bs_ship_deep(hess, xn, yn, h, X, Y, Xa, Xb, Ya, Yb, a, b);
                 }
-                taken = bs_step_ship<AXIS>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b);
+                if (!taken) {
+                    double xs = XX_last, ys = YY_last;
+                    if (!has_sums) {
+                        xs = (d_is0(X) & !d_is0(xn)) ? xn : d_add_here(X, xn);
+                        ys = (d_is0(Y) & !d_is0(yn)) ? yn : d_add_here(Y, yn);
+                    }
+                    taken = bs_step_ship<AXIS>(hess, xn, yn, h, X, Y, xs, ys, Xa, Xb, Ya, Yb, a, b);
+                }
             }
             if (!taken) {
                 if (hess) bs_hess<T>(flavor, h, xn, yn, X, Y, Xa, Xb, Ya, Yb);
@@ -1187,10 +1336,8 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
         BSRef<T>::orbit(R, w, Xs, Ys);
         T XX, YY;
         if constexpr (IsDouble<T>::value) {
-            // a sum with 0 is its other term while that is not 0
-            XX = xn; YY = yn;
-            if (!d_is0(Xs) | d_is0(xn)) XX = d_add_here(xn, Xs);
-            if (!d_is0(Ys) | d_is0(yn)) YY = d_add_here(yn, Ys);
+            XX = d_add_far(xn, Xs);
+            YY = d_add_far(yn, Ys);
             XX_last = XX; YY_last = YY;
             has_sums = true;
         } else {
@@ -1209,7 +1356,8 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
             if (hess) {
                 T Ha, Hb, Hc, Hd;
                 BSRef<T>::hess(R, w, Ha, Hb, Hc, Hd);
-                h[0] += Ha; h[1] += Hb; h[2] += Hc; h[3] += Hd;
+                h[0] = bs_add<T, FL>(h[0], Ha); h[1] = bs_add<T, FL>(h[1], Hb);
+                h[2] = bs_add<T, FL>(h[2], Hc); h[3] = bs_add<T, FL>(h[3], Hd);
             }
             w = 0; nreb++; continue;
         }
@@ -1220,7 +1368,8 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
             if (hess) {
                 T Ha, Hb, Hc, Hd;
                 BSRef<T>::hess(R, w, Ha, Hb, Hc, Hd);
-                h[0] += Ha; h[1] += Hb; h[2] += Hc; h[3] += Hd;
+                h[0] = bs_add<T, FL>(h[0], Ha); h[1] = bs_add<T, FL>(h[1], Hb);
+                h[2] = bs_add<T, FL>(h[2], Hc); h[3] = bs_add<T, FL>(h[3], Hd);
             }
             w = 0; nreb++; continue;
         }
@@ -1287,8 +1436,9 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
 // iterations, takes 45.5 ms so, 48.0 with three blocks, 48.9 with five, 60.6 with
 // two), flavor 5 three (its views spend more in the fr steps, which spill: 31 to 34
 // ms, 35 with four); the others two (128): flavor 1 in the double form, 255^2 pixels
-// of the period-12 nucleus to 20000 iterations, takes 67 ms with them, 95 ms at
-// its own 156 registers and one block, 73 ms at 80 with spills
+// of the period-12 nucleus to 20000 iterations, took 68 ms with them before
+// bs_ship_deep (39 with it), 95 ms at its own 156 registers and one block, 73 ms at
+// 80 with spills
 template <class T, int FL, bool AXIS>
 __global__ void __launch_bounds__(256, IsFr<T>::value ? (FL == 5 ? 3 : 4) : 2)
 k_perturb_bs(WorkDev W, CalcDev C) {

@@ -237,6 +237,16 @@ FSG_DEV xc frame_add(double2 p, int ep, double2 q, int eq, bool &ok) {
     ok &= ((unsigned)(qy + d - 1) < 2045u) | d_is0(q.y);
     return xc_make(p.x + d_shift(q.x, d), p.y + d_shift(q.y, d), ep);
 }
+// a + b, with a sum only where one takes part in the other: 56 binary orders
+// apart (or beside a zero or a subnormal) the larger is the sum; two zeros add to
+// -0 where both are
+FSG_DEV double d_add_far(double a, double b) {
+    const int g = d_field(a) - d_field(b);
+    if (g >= 56) return a;
+    if (g <= -56) return b;
+    if (d_is0(a) & d_is0(b)) return d_zero(((d_hi(a) & d_hi(b)) >> 31) != 0u);
+    return d_add_here(a, b);
+}
 // the larger part's exponent field (0 for zero and subnormal parts)
 FSG_DEV int d_field_max(double2 z) { return max(d_field(z.x), d_field(z.y)); }
 FSG_DEV int d_field_min(double2 z) { return min(d_field(z.x), d_field(z.y)); }
