@@ -950,8 +950,12 @@ FSG_DEV double d_two_far(double a1, double b1, double a2, double b2, bool minus)
     return d_add_far(d_mul_here(a1, b1), d_flip(d_mul_here(a2, b2), flip));
 }
 
-// the exponent field of x, far below any for 0
-FSG_DEV int d_field0(double x) { return d_is0(x) ? -20000 : d_field(x); }
+// the exponent field of x, continued below 1 for subnormals, far below any for 0
+FSG_DEV int d_field0(double x) {
+    const int f = d_field(x);
+    if (f != 0) return f;
+    return d_is0(x) ? -20000 : 12 - __clzll((long long)(dbits(x) << 1 >> 1));
+}
 // signs of products as words whose top bit counts
 FSG_DEV unsigned d_sgn2(double a, double b) { return d_hi(a) ^ d_hi(b); }
 FSG_DEV double d_zero_of(unsigned s) { return d_zero((s >> 31) != 0u); }
@@ -1004,11 +1008,10 @@ FSG_DEV bool bs_ship_crit(bool hess, double &xn, double &yn, double h[4], double
 // that they enter, so neither they nor the sums are taken.  Exponent fields say
 // so for each sum (a product's exponent is the sum of its factors', or one more;
 // `far` binary orders leave a power of two its ulp): 10 products and 6 sums
-// remain of 18 and 15, which the FP64 pipe takes: a product there is one
-// instruction where the integer pipes take thirty, and the pipe is no longer what
-// bounds the loop (with two of the ten as integer products 8 % longer).  255^2
-// pixels of the period-12 nucleus to 20000 iterations: 67 ms without this step and
-// bs_ship_crit, 39 with them.  Yz, Xb, Ya: zeros, for the signs of results that are 0
+// remain of 18 and 15.  The integer pipes take four of the products: 255^2 pixels
+// of the period-12 nucleus to 20000 iterations take 35.7 ms with four or six of
+// them there, 37.2 with two, 39.3 with none, 67 without this step and
+// bs_ship_crit.  Yz, Xb, Ya: zeros, for the signs of results that are 0
 // because all their terms are.  false (nothing changed) where a sum is open.
 FSG_DEV bool bs_ship_deep(bool hess, double &xn, double &yn, double h[4], double X, double Yz, double Xa,
                           double Xb, double Ya, double Yb, double a, double b) {
@@ -1019,6 +1022,11 @@ FSG_DEV bool bs_ship_deep(bool hess, double &xn, double &yn, double h[4], double
     bool ok = (fX - max(x, y) >= far + 3) & (min(x, y) >= 1) & (min(x, y) + fX >= 1025)
               & (x + fX >= 2 * y + 2 + far);                 // yn yn beside xn (xn + 2 X)
     const unsigned s1 = d_sgn2(yn, X) & 0x80000000u;
+    if (!ok) return false;
+    const dfac dX = dfac_of(X);
+    dfac dX2 = dX;
+    dX2.s += 0x00100000u;
+    const double px = dfac_mul(dfac_of(xn), dX2, ok), op = dfac_mul(dfac_of(yn), dX, ok);
     double n0 = 0., n1 = 0., n2 = 0., n3 = 0.;
     if (hess) {
         // exponents of da = ((xa yn + xn ya) + ya X) + yn Xa and of
@@ -1028,47 +1036,65 @@ FSG_DEV bool bs_ship_deep(bool hess, double &xn, double &yn, double h[4], double
         const int fXa = d_field(Xa), fYb = d_field(Yb);
         const int sa = max(xa + y, x + ya) + 2, ta = ya + fX, ua = y + fXa;
         const int sb = max(xb + y, x + yb) + 2, tb = x + fYb, ub = yb + fX;
-        const bool a3 = ya >= 1 && ta - sa >= far, b3 = tb - sb >= far;
+        const bool a3 = ta - sa >= far, b3 = tb - sb >= far;
         ok &= (min(fXa, fYb) >= 1)
               & (max(max(max(xa, xb), max(ya, yb)), max(max(fXa, fYb), fX)) <= 1900);
         ok &= a3 | (ua - max(sa, ta + 2) >= far + 1);
-        ok &= b3 | ((yb >= 1) & (ub - max(sb, tb + 2) >= far + 1));
+        ok &= b3 | (ub - max(sb, tb + 2) >= far + 1);
         if (!ok) return false;
         n2 = d_mul_here(yn, Xa);
-        n3 = d_mul_here(gb, X);
+        double gx;
+        if (min(ya, yb) + fX >= 1025) {
+            gx = dfac_mul(dfac_of(ga), dX, ok);
+            n3 = dfac_mul(dfac_of(gb), dX, ok);
+            if (!ok) return false;
+        } else {
+            gx = d_mul_here(ga, X);
+            n3 = d_mul_here(gb, X);
+        }
         n0 = d_mul_here(Xa, xn);
         n1 = d_mul_here(Yb, yn);                 // vb = yn yb + Yb yn
         if (fYb - yb < far + 2) n1 = d_add_here(d_mul_here(yn, gb), n1);
         n1 = d_flip(d_twice(n1), 0x80000000u);
-        if (a3) n2 = d_add_here(d_mul_here(ga, X), n2);
+        if (a3) n2 = d_add_here(gx, n2);
         if (b3) n3 = d_add_here(d_mul_here(xn, Yb), n3);
         n0 = d_add_here(d_mul_here(X, ha), n0);
         n1 = d_add_here(d_twice(d_mul_here(X, hb)), n1);
         // va = yn ya
-        if (!((d_field(n0) >= max(y + ya - 1023 + 2 + far, 1)) | (d_is0(n0) & (y + ya <= 968)))) return false;
+        if (!((d_field(n0) >= max(y + ya - 1023 + 2 + far, 1)) | (y + ya <= 968))) return false;
         n0 = d_twice(n0);
+        if (s1) n3 = d_add_here(d_twice(d_mul_here(X, Yb)), n3);
         if (d_is0(n0) | d_is0(n1) | d_is0(n2) | d_is0(n3)) {
-            // with every term of the Hessian's steps underflowing: their signs
-            if (max(max(xa, xb), max(ya, yb)) + 1 + fX > 968 || max(ua, tb) > 968 || y + fYb > 968 || x + fXa > 968)
-                return false;
-            const unsigned pa = d_sgn2(ha, yn) & d_sgn2(xn, ga) & d_sgn2(ha, Yz) & d_sgn2(xn, Ya) & d_sgn2(ga, X) & d_sgn2(yn, Xa);
-            const unsigned pb = d_sgn2(hb, yn) & d_sgn2(xn, gb) & d_sgn2(hb, Yz) & d_sgn2(xn, Yb) & d_sgn2(gb, X) & d_sgn2(yn, Xb);
+            // a sum whose terms all underflow has the sign that their zeros add to
+            const bool x3 = d_is0(n3);
+            const unsigned pa = d_sgn2(ha, yn) & d_sgn2(xn, ga) & d_sgn2(ha, Yz) & d_sgn2(xn, Ya)
+                                & d_sgn2(ga, X) & d_sgn2(yn, Xa);
+            const unsigned pb = d_sgn2(hb, yn) & d_sgn2(xn, gb) & d_sgn2(hb, Yz) & d_sgn2(xn, Yb)
+                                & d_sgn2(gb, X) & d_sgn2(yn, Xb);
             const unsigned da = d_sgn2(Xa, Yz) & d_sgn2(X, Ya), db = d_sgn2(X, Yb);
-            n0 = d_zero_of(d_sgn2(X, ha) & d_sgn2(Xa, xn) & ~(d_sgn2(yn, ga) & d_sgn2(Ya, yn)));
-            n1 = d_zero_of(d_sgn2(X, hb) & d_sgn2(Xb, xn) & ~(d_sgn2(yn, gb) & d_sgn2(Yb, yn)));
-            // ddiffabsdX (0 or -2) times the reference's d(XY), and ddiffabsdx times this
-            n2 = d_zero_of(s1 ? ~da & ~pa : da & pa);
-            n3 = s1 ? d_twice(d_mul_here(X, Yb)) : d_zero_of(db & pb);
-            h[0] = n0; h[1] = n1; h[2] = n2; h[3] = s1 ? d_twice(d_flip(n3, s1)) : n3;
-        } else {
-            if (s1) n3 = d_add_here(d_twice(d_mul_here(X, Yb)), n3);
-            if (min(min(d_field(n1), d_field(n2)), d_field(n3)) < 1) return false;
-            h[0] = n0; h[1] = n1; h[2] = d_twice(d_flip(n2, s1)); h[3] = d_twice(d_flip(n3, s1));
+            if (d_is0(n0)) {
+                if (!(d_is0(d_mul_here(X, ha)) & d_is0(d_mul_here(Xa, xn)))) return false;
+                n0 = d_zero_of(d_sgn2(X, ha) & d_sgn2(Xa, xn) & ~(d_sgn2(yn, ga) & d_sgn2(Ya, yn)));
+            }
+            if (d_is0(n1)) {
+                if (!(d_is0(d_mul_here(X, hb)) & d_is0(d_mul_here(Yb, yn)) & d_is0(d_mul_here(yn, gb)))) return false;
+                n1 = d_zero_of(d_sgn2(X, hb) & d_sgn2(Xb, xn) & ~(d_sgn2(yn, gb) & d_sgn2(Yb, yn)));
+            }
+            if (d_is0(n2)) {
+                if (!(d_is0(d_mul_here(ga, X)) & d_is0(d_mul_here(yn, Xa)))) return false;
+                // ddiffabsdX (0 or -2) times the reference's d(XY), and ddiffabsdx times this
+                n2 = d_flip(d_zero_of(s1 ? ~da & ~pa : da & pa), s1);
+            }
+            if (x3) {
+                if ((s1 != 0u) | !(d_is0(d_mul_here(gb, X)) & d_is0(d_mul_here(xn, Yb)))) return false;
+                n3 = d_zero_of(db & pb);
+            }
         }
+        h[0] = n0; h[1] = n1; h[2] = d_twice(d_flip(n2, s1)); h[3] = d_twice(d_flip(n3, s1));
     }
     if (!ok) return false;
-    xn = d_add_here(d_mul_here(xn, d_twice(X)), a);
-    yn = d_add_here(d_twice(d_flip(d_mul_here(yn, X), s1)), d_flip(b, 0x80000000u));
+    xn = d_add_here(px, a);
+    yn = d_add_here(d_twice(d_flip(op, s1)), d_flip(b, 0x80000000u));
     return true;
 }
 
@@ -1437,7 +1463,7 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
 // two), flavor 5 three (its views spend more in the fr steps, which spill: 31 to 34
 // ms, 35 with four); the others two (128): flavor 1 in the double form, 255^2 pixels
 // of the period-12 nucleus to 20000 iterations, took 68 ms with them before
-// bs_ship_deep (39 with it), 95 ms at its own 156 registers and one block, 73 ms at
+// bs_ship_deep (36 with it), 95 ms at its own 156 registers and one block, 73 ms at
 // 80 with spills
 template <class T, int FL, bool AXIS>
 __global__ void __launch_bounds__(256, IsFr<T>::value ? (FL == 5 ? 3 : 4) : 2)
