@@ -1,7 +1,7 @@
 // fsg_bs.cuh -- the Burning Ship family perturbation loop, templated on the
 // real type of the deltas:
 //   * double -- the reference's standard branch (instantiated in
-//     fsg_perturb.cu, compiled without FMA contraction: one rounding per
+//     fsg_perturb_bs64.cu, compiled without FMA contraction: one rounding per
 //     operation in the order of the reference source);
 //   * fr -- FP32 mantissa + int32 exponent (instantiated in fsg_perturb_bs32.cu):
 //     no underflow at any depth and FP32-pipe arithmetic instead of GB300's

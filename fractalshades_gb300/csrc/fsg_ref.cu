@@ -5,8 +5,8 @@
 //     models/mandelbrot_Mn.py:645-652),
 //     numba_dZndz_path (:2466-2516), numba_dZndc_path_BS + incr_deriv_ref_BS
 //     (:2339-2463).  These are first-order linear recurrences evaluated in
-//     the reference's order by one thread (they are O(len) and run once per
-//     reference);
+//     the reference's order, one step after the other (they are O(len) and run
+//     once per reference);
 //   * the compressed BLA tree: numba_make_BLA (:1819-1881) / numba_make_BLA_BS
 //     (:1884-1973) with combine_BLA (:1983-2024) / combine_BLA_BS
 //     (:2027-2105).  The 8-iteration leaves are built one compressed block per

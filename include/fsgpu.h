@@ -126,9 +126,12 @@ typedef struct {
                                  mandelbrot_Mn.py:325-333)                    */
     int32_t block;            /* launch shape (chosen by the autotuner,
                                  fractalshades_gb300/tune.py): threads per
-                                 CTA, 0 = the kernel's default (256; 128 for
-                                 the FE32 power-2 kernel), else a multiple of
-                                 32 up to that default                        */
+                                 CTA, 0 = the launcher's choice (128 for the
+                                 FE32 power-2 kernel; else 256, or 64 where the
+                                 FP64, XR64 and standard launchers see that the
+                                 SMs hold the whole image at once), else a
+                                 multiple of 32 up to the kernel's bound (256;
+                                 128 for the FE32 power-2 kernel)             */
     int32_t ctas_per_sm;      /* resident CTAs per SM of the persistent grid,
                                  0 = the occupancy limit, else at most that
                                  many (the allocation-free entry point keeps
