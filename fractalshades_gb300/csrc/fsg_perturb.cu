@@ -246,10 +246,9 @@ __device__ __forceinline__ bool dz_below(double2 Z, double2 z, int e) {
 // on the frame, so the frames of this loop differ from the reference's lazily
 // normalised ones (frame_add).  Whatever leaves the ranges those forms need
 // takes the reference's step, operation by operation.
-template <bool XR>
+template <bool XR, class Count>
 __device__ __forceinline__ void pixel_m2_fast(const TileDev &T, const CalcDev &C, long long ip,
-                                              unsigned long long &nfull, unsigned long long &nbla,
-                                              unsigned long long &nreb, unsigned long long &itsum) {
+                                              Count &nfull, Count &nbla, Count &nreb, Count &itsum) {
     const RefDev &R = *T.ref;
     const long long np = (long long)T.nx * T.ny;
     const bool dzndz_on = C.interior, dzndc_on = C.calc_dzndc;
@@ -499,7 +498,7 @@ __device__ __forceinline__ void pixel_m2_fast(const TileDev &T, const CalcDev &C
     T.stop_iter[ip] = n;
     T.stop_reason[ip] = stop;
     fsg_epilogue(T, C, ip, zn, hypot(dzndc.x, dzndc.y), n);
-    itsum += (unsigned long long)n;
+    itsum += (Count)n;
 }
 
 template <bool XR, bool MN, bool ORB>
@@ -520,12 +519,51 @@ __global__ void __launch_bounds__(256) k_perturb_m2(WorkDev W, CalcDev C) {
     fsg_flush_stats(W, itsum, nfull, nbla, nreb);
 }
 
+// The Xrange power-2 loop at three CTAs of 256 an SM (80 registers, with spills)
+// instead of two (123): the latency of its chains bounds it.  513 x 511 pixels of
+// the period-2562 nucleus take 10.0 ms so and 10.8 with two, 300 x 300 (one wave of
+// three, two of two) 22 % less.  The statistics are 32-bit per pixel and summed in
+// shared memory, where 64-bit sums would hold 8 registers in the loop (10.3 ms).
+__global__ void __launch_bounds__(256, 3) k_perturb_m2_xr_dense(WorkDev W, CalcDev C) {
+    extern __shared__ unsigned long long m2_smem[];            // sized at launch
+    unsigned long long *acc = m2_smem + threadIdx.x;           // acc[k * blockDim.x]
+    long long *s_start = (long long *)(m2_smem + 4 * blockDim.x);
+    const int nb = blockDim.x;
+    for (int k = 0; k < 4; k++) acc[k * nb] = 0ULL;
+    fsg_load_starts(W, s_start);
+    int t; long long ip;
+    while (true) {
+        if (!fsg_claim_poll(W, s_start, t, ip)) break;
+        unsigned nfull = 0, nbla = 0, nreb = 0, n = 0;
+        pixel_m2_fast<true>(W.tiles[t], C, ip, nfull, nbla, nreb, n);
+        fsg_account(W, (unsigned long long)n);
+        acc[0] += n;
+        acc[nb] += nfull;
+        acc[2 * nb] += nbla;
+        acc[3 * nb] += nreb;
+    }
+    fsg_flush_stats(W, acc[0], acc[nb], acc[2 * nb], acc[3 * nb]);
+}
+
 template <bool XR, bool MN, bool ORB>
 static void launch_m2(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s) {
     const size_t sm = fsg_starts_smem(W);
-    block = fsg_fp64_block(k_perturb_m2<XR, MN, ORB>, block, W.total - W.base, sm);
-    k_perturb_m2<XR, MN, ORB><<<fsg_auto_grid(k_perturb_m2<XR, MN, ORB>, grid, block,
-                                              W.total - W.base, sm), block, sm, s>>>(W, C);
+    const long long total = W.total - W.base;
+    if constexpr (XR && !MN && !ORB) {
+        // Images that two CTAs an SM do not hold at once; smaller ones, and interior
+        // detection, take 4 to 7 % longer with three.
+        const long long two = 256LL * fsg_auto_grid(k_perturb_m2<XR, MN, ORB>, 0, 256, 1LL << 40, sm);
+        if (!C.interior && total > two) {
+            const size_t acc = 4 * sizeof(unsigned long long);      // per thread
+            const int b = fsg_fp64_block(k_perturb_m2_xr_dense, block, total, sm + 256 * acc);
+            const size_t smd = sm + acc * (size_t)b;
+            k_perturb_m2_xr_dense<<<fsg_auto_grid(k_perturb_m2_xr_dense, grid, b, total, smd), b, smd, s>>>(W, C);
+            return;
+        }
+    }
+    block = fsg_fp64_block(k_perturb_m2<XR, MN, ORB>, block, total, sm);
+    k_perturb_m2<XR, MN, ORB><<<fsg_auto_grid(k_perturb_m2<XR, MN, ORB>, grid, block, total, sm), block, sm,
+                                s>>>(W, C);
 }
 
 template <bool ORB>

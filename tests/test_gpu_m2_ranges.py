@@ -147,3 +147,21 @@ def test_fe32_escape_radius(ctx, M):
     # step more or less, which a few steps of squaring make rare
     off = si[0] - si0[0] != more
     assert off.sum() <= 0.01 * off.size and np.abs(si[0] - si0[0] - more).max() <= 1
+
+
+@pytest.mark.parametrize("nx,ny", [(283, 275), (331, 353), (411, 397)])
+def test_xr64_images_above_two_ctas_an_sm(ctx, nx, ny):
+    """Images that two CTAs an SM do not hold at once run in the Xrange loop's
+    three-CTA kernel: the pixels of a smaller launch, and its statistics."""
+    w = _view("bulb", "1e-305", True, nx=nx, ny=ny, max_iter=1200)
+    ref = _reference(ctx, w, False)
+    a = _run(ctx, w, ref, "xr64")
+    big = ctx.stats()
+    xs, ys = w.xs, w.ys
+    cut = 100
+    w.nx, w.ny, w.xs, w.ys = cut, cut, xs[:cut], ys[:cut]
+    b = _run(ctx, w, ref, "xr64")
+    for x, y in zip(a, b):
+        assert np.array_equal(x.reshape(x.shape[0], ny, nx)[:, :cut, :cut], y.reshape(y.shape[0], cut, cut))
+    assert big["pixels"] == nx * ny and big["pixel_iters"] == a[1].sum()
+    assert 0 < big["full_steps"] <= big["pixel_iters"]
