@@ -1456,17 +1456,19 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
     return n;
 }
 
-// The FP32 + exponent kernels hold four 256-thread blocks per SM (at most 64
-// registers a thread: short chains of FP32 and integer operations want warps more
-// than registers -- flavor 1, 640^2 pixels of a period-3 nucleus to 20000
-// iterations, takes 45.5 ms so, 48.0 with three blocks, 48.9 with five, 60.6 with
-// two), flavor 5 three (its views spend more in the fr steps, which spill: 31 to 34
-// ms, 35 with four); the others two (128): flavor 1 in the double form, 255^2 pixels
-// of the period-12 nucleus to 20000 iterations, took 68 ms with them before
-// bs_ship_deep (36 with it), 95 ms at its own 156 registers and one block, 73 ms at
-// 80 with spills
-template <class T, int FL, bool AXIS>
-__global__ void __launch_bounds__(256, IsFr<T>::value ? (FL == 5 ? 3 : 4) : 2)
+// DENSE: the FP32 + exponent kernels hold three 256-thread blocks per SM (at most 85
+// registers a thread), or four (64, with spills) for images that three do not hold
+// at once: short chains of FP32 and integer operations want warps more than
+// registers -- flavor 1, 640^2 pixels of a period-3 nucleus to 20000 iterations,
+// takes 45.5 ms with four, 48.0 with three, 48.9 with five, 60.6 with two; images of
+// 150^2 and 300^2 take 1 to 5 % longer with four, of 450^2 and 600^2 5 to 14 % less,
+// but for flavor 5, whose views spend more in the fr steps, which spill (31 to 34
+// ms with three, 35 with four).  The other kernels hold two (128): flavor 1 in the
+// double form, 255^2 pixels of the period-12 nucleus to 20000 iterations, took 68 ms
+// with them before bs_ship_deep (36 with it), 95 ms at its own 156 registers and one
+// block, 73 ms at 80 with spills
+template <class T, int FL, bool AXIS, bool DENSE>
+__global__ void __launch_bounds__(256, DENSE ? 4 : IsFr<T>::value ? 3 : 2)
 k_perturb_bs(WorkDev W, CalcDev C) {
     // sized at launch: per-thread statistics (64-bit sums would hold 8 registers
     // in the loop), then the pixel offsets of the launch's tiles

@@ -96,3 +96,32 @@ def test_bs_real_reference_alone_and_in_a_mixed_launch(ctx, mode, width, hess):
 
     for a, b in zip(run([0])[0], run([0, 1])[0]):
         assert np.array_equal(a, b, equal_nan=a.dtype == np.float64)
+
+
+@pytest.mark.parametrize("seed", [4, 5])
+@pytest.mark.parametrize("flavor", [1, 2, 3, 4, 5])
+def test_bs_fe32_images_above_three_ctas_an_sm(ctx, flavor, seed):
+    """Images that three CTAs an SM do not hold at once run in the four-CTA
+    kernel: the pixels of a smaller launch."""
+    import mpmath
+    from fractalshades_gb300 import _native as nat
+    t = syn.config4_workload(seed=seed, n_tiles=1, max_iter=300, kind=flavor)[0]
+    dx = fsx.mpf_to_Xrange(mpmath.mpf("1e-8"))
+    ref = nat.Reference(ctx, t.Zn, div_iter=t.div_iter, order=t.ref_order, flavor=flavor,
+                        calc_dzndc=True, scale_m=dx.m, scale_e=dx.e, bla=True,
+                        kc=float(np.ldexp(dx.m, dx.e)), bla_eps=1e-6)
+    xs, ys = syn.image_axes(353, 347)
+
+    def run(xs, ys):
+        n = xs.size * ys.size
+        Z, sr = np.zeros((6, n)), -np.ones((1, n), dtype=np.int8)
+        si = np.zeros((1, n), dtype=np.int32)
+        tile = nat.make_tile(xs=xs, ys=ys, lin_mat=LIN, Z=Z, stop_reason=sr, stop_iter=si, ref=ref,
+                             dx_m=dx.m, dx_e=dx.e, drift_m=0.01 * dx.m, drift_e=dx.e,
+                             drifty_m=0., drifty_e=0)
+        ctx.perturb_tiles(nat.make_calc(max_iter=300, M_divergence=1000., flavor=flavor,
+                                        calc_dzndc=True, bla=True, mode="fe32"), [tile])
+        return [x.reshape(x.shape[0], ys.size, xs.size) for x in (Z, sr, si)]
+
+    for big, small in zip(run(xs, ys), run(xs[:90], ys[:70])):
+        assert np.array_equal(big[:, :70, :90], small, equal_nan=small.dtype == np.float64)
