@@ -1459,7 +1459,7 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
 // DENSE: the FP32 + exponent kernels hold three 256-thread blocks per SM (at most 85
 // registers a thread), or four (64, with spills) for images that three do not hold
 // at once: short chains of FP32 and integer operations want warps more than
-// registers -- flavor 1, 640^2 pixels of a period-3 nucleus to 20000 iterations,
+// registers -- flavor 1, 640^2 pixels of a period-12 nucleus to 20000 iterations,
 // takes 45.5 ms with four, 48.0 with three, 48.9 with five, 60.6 with two; images of
 // 150^2 and 300^2 take 1 to 5 % longer with four, of 450^2 and 600^2 5 to 14 % less,
 // but for flavor 5, whose views spend more in the fr steps, which spill (31 to 34

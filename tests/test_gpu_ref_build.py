@@ -64,3 +64,40 @@ def test_tables_beside_a_path_and_alone(ctx, n, flavor, mode):
     b = _image(ctx, derived, flavor, mode, 0.25 + 0.125j)
     for x, y in zip(a, b):
         assert np.array_equal(x.view(np.uint8), y.view(np.uint8))
+
+
+@pytest.mark.parametrize("flavor", [0, 1])
+def test_tables_of_many_live_references(ctx, flavor):
+    """Tables that share blocks of a context's pool do not touch: every
+    reference of a set built, partly freed and built again holds the tables it
+    holds alone."""
+    from fractalshades_gb300 import _native as nat
+    lens = [3, 9, 17, 100, 257, 1000, 4095, 4096, 4097, 20000]
+    names = ("dzndc", "bla") if flavor == 0 else ("bs_paths", "bla")
+
+    def build(c, n):
+        return nat.Reference(c, _orbit(n, n), div_iter=10 ** 6, order=n, flavor=flavor, scale_m=1.25,
+                             scale_e=-40, calc_dzndc=True, bla=True, kc=float(np.ldexp(1.25, -40)))
+
+    def tables(ref, n):
+        out = []
+        for k in names:
+            if k == "bla" and n < 8:
+                continue
+            t = ref.download(k)
+            out += list(t) if isinstance(t, tuple) else [t]
+        return [np.ascontiguousarray(x).view(np.uint8) for x in out if x is not None]
+
+    live = {n: build(ctx, n) for n in lens}
+    for n in lens[::2]:
+        live[n].free()
+        live[n] = build(ctx, n)
+    other = nat.Context(0)
+    for n in lens:
+        alone = build(other, n)
+        for a, b in zip(tables(live[n], n), tables(alone, n)):
+            assert np.array_equal(a, b)
+        alone.free()
+    other.close()
+    for r in live.values():
+        r.free()
