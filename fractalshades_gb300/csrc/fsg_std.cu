@@ -28,8 +28,9 @@ __device__ __forceinline__ double2 std_c(const TileDev &T, long long ip) {
 //   start: c known, the state of z_0 = 0 in place (n = 0); takes the first
 //          steps of an ordinary pixel (all lanes of a warp run it together);
 //   step:  one iteration; products by fsg_soft.cuh, and by the multiplies
-//          (step_full, the reference's operations one by one) where those
-//          leave the step open;
+//          (step_full, the reference's operations one by one, out of line)
+//          where a factor is out of their range (in_range) or a product is left
+//          open;
 //   stop:  the tests after it: the stop reason, -1 to go on;
 //   store: the outputs.
 // OPT: the optional outputs d2zndc2 (mandelbrot_M2.py:316-317) and the orbit
@@ -46,6 +47,12 @@ __device__ __forceinline__ void std_opt_take(StdOpt<OPT> &o, const CalcDev &C, i
     if constexpr (OPT) { if (C.backshift > 0) o.S.take(n, C.backshift, z); }
 }
 
+template <class Mdl>
+static __device__ __noinline__ typename Mdl::Px std_step_full(typename Mdl::Px p, const CalcDev &C) {
+    Mdl::step_full(p, C);
+    return p;
+}
+
 struct CoopLane { unsigned k, neg; bool add; double g; };
 
 // Power-2 and power-n Mandelbrot: the complex state
@@ -58,6 +65,11 @@ struct StdMandel {
     static __device__ __forceinline__ void init(Px &p, const CalcDev &C, double2 c) {
         p.c = c; p.zn = cx(0., 0.); p.dzndz = p.zn; p.dzndc = p.zn; p.n = 0;
         std_opt_init<OPT>(p.o, C);
+    }
+    static __device__ __forceinline__ bool in_range(const Px &p, const CalcDev &C) {
+        bool ok = dfac_ok(p.zn) & dfac_ok(p.dzndz) & dfac_ok(p.dzndc);
+        if constexpr (OPT) { if (C.d2) ok &= dfac_ok(p.o.d2); }
+        return ok;
     }
     static __device__ __forceinline__ int stop(const Px &p, const CalcDev &C) {
         if (fsg_escaped(C, p.zn)) return 1;
@@ -75,14 +87,13 @@ struct StdMandel {
 template <bool OPT>
 struct StdM2 : StdMandel<OPT> {
     typedef StdPx<OPT> Px;
-    static __device__ __noinline__ Px step_full(Px p, const CalcDev &C) {
+    static __device__ __forceinline__ void step_full(Px &p, const CalcDev &C) {
         if constexpr (OPT) {
             if (C.d2) p.o.d2 = rmul2(cadd(cmul(p.o.d2, p.zn), csq(p.dzndc)));
         }
         p.dzndc = caddr(cmul(rmul2(p.dzndc), p.zn), 1.);
         p.dzndz = cmul(rmul2(p.dzndz), p.zn);
         p.zn = cadd(csq(p.zn), p.c);
-        return p;
     }
     static __device__ __forceinline__ void step(Px &p, const CalcDev &C) {
         bool ok = dfac_ok(p.zn) & dfac_ok(p.dzndz) & dfac_ok(p.dzndc);
@@ -102,24 +113,23 @@ struct StdM2 : StdMandel<OPT> {
             p.zn = cadd(sq, p.c); p.dzndz = dz; p.dzndc = dc;
             if constexpr (OPT) { if (C.d2) p.o.d2 = d2; }
         } else {
-            p = step_full(p, C);
+            p = std_step_full<StdM2<OPT>>(p, C);
         }
     }
     // z_1 = c and dz_1 = dc_1 = 1, z_2 = c^2 + c, dz_2 = 2 c and dc_2 = 2 c + 1
     // for c in the range of the integer products (elsewhere the pixel starts at
-    // n = 0); with d2zndc2 three plain steps
+    // n = 0); with d2zndc2 up to three plain steps, those before the last one
     static __device__ __forceinline__ void start(Px &p, const CalcDev &C) {
         Px s = p;
         if (OPT && C.d2) {
-            bool go = C.max_iter > 3;
-            for (int n = 1; n <= 3 && go; n++) {
-                s = step_full(s, C);
+            for (int n = 1; n <= min(3, C.max_iter - 1); n++) {
+                step_full(s, C);
                 if (n == 1) s.dzndz = cx(1., 0.);
                 std_opt_take<OPT>(s.o, C, n, s.zn);
-                go = StdMandel<OPT>::stop(s, C) < 0;
+                if (StdMandel<OPT>::stop(s, C) >= 0) break;
+                s.n = n;
+                p = s;
             }
-            s.n = 3;
-            if (go) p = s;
             return;
         }
         bool ok = dfac_ok(p.c) && C.max_iter > 2;
@@ -139,6 +149,7 @@ struct StdM2 : StdMandel<OPT> {
     // and its partner `pr`, the other part of its pair.  Every component is
     // own x -+ pr y (doubled for the derivatives), and what is added to it.
     static constexpr bool kCoop = !OPT;
+    static constexpr bool kPlain = OPT;                  // std_plain_chunk
     static __device__ __forceinline__ double coop_get(const Px &p, int role) {
         return role == 0 ? p.zn.x : role == 1 ? p.zn.y : role == 2 ? p.dzndz.x
                : role == 3 ? p.dzndz.y : role == 4 ? p.dzndc.x : p.dzndc.y;
@@ -165,7 +176,8 @@ struct StdM2 : StdMandel<OPT> {
     }
     // step_full for one lane
     static __device__ __forceinline__ double coop_full(double own, double pr, double x, double y,
-                                                       const Px &p, const CalcDev &, int role, int n) {
+                                                       const Px &p, const CoopLane &, const CalcDev &,
+                                                       int role, int n) {
         const bool im = role & 1;
         double2 a = im ? cx(pr, own) : cx(own, pr);
         if (role >= 2) a = rmul2(a);
@@ -241,7 +253,8 @@ template <bool OPT>
 struct StdMn : StdMandel<OPT> {
     typedef StdPx<OPT> Px;
     static constexpr bool kCoop = false;
-    static __device__ __noinline__ Px step_full(Px p, const CalcDev &C) {
+    static constexpr bool kPlain = true;
+    static __device__ __forceinline__ void step_full(Px &p, const CalcDev &C) {
         const int nexp = C.nexp;
         const double deg = (double)nexp;
         double2 zm1, zm;
@@ -265,7 +278,6 @@ struct StdMn : StdMandel<OPT> {
         p.dzndc = caddr(cmul(rmul(deg, p.dzndc), zm1), 1.);
         p.dzndz = cmul(rmul(deg, p.dzndz), zm1);
         p.zn = cadd(zm, p.c);
-        return p;
     }
     // deg * z by the integer products (by a small integer: ties are common)
     static __device__ __forceinline__ double2 scaled(const dfac &deg, double2 z) {
@@ -292,8 +304,14 @@ struct StdMn : StdMandel<OPT> {
                                        cfac_mul(cfac_of(v), cfac_of(zm2), ok));
                 ok &= dfac_ok(w);
                 d2 = scaled(deg, w);
+            } else if (C.d2) {
+                // n = 2: z^0 = 1 leaves its factors as they are
+                ok &= dfac_ok(p.o.d2);
+                const double2 w = cadd(cfac_mul(cfac_of(p.o.d2), cfac_of(p.zn), ok),
+                                       cfac_mul(cfac_of(p.dzndz), cfac_of(p.dzndc), ok));
+                ok &= dfac_ok(w);
+                d2 = scaled(deg, w);
             }
-            ok &= (d2_on || !C.d2);
         }
         if (!d2_on) zm1 = ipow_soft(p.zn, nexp - 1, ok);
         ok &= dfac_ok(zm1);
@@ -306,25 +324,24 @@ struct StdMn : StdMandel<OPT> {
         const double2 dz = cfac_mul(cfac_of(ez), fm, ok);
         if (ok) {
             p.zn = cadd(zm, p.c); p.dzndz = dz; p.dzndc = dc;
-            if constexpr (OPT) { if (d2_on) p.o.d2 = d2; }
+            if constexpr (OPT) { if (C.d2) p.o.d2 = d2; }
         } else {
-            p = step_full(p, C);
+            p = std_step_full<StdMn<OPT>>(p, C);
         }
     }
     // z_1 = c, dz_1 = dc_1 = 1; dz_2 = n c^(n-1), dc_2 = dz_2 + 1,
-    // z_2 = c^n + c; with d2zndc2 three plain steps
+    // z_2 = c^n + c; with d2zndc2 up to three plain steps
     static __device__ __forceinline__ void start(Px &p, const CalcDev &C) {
         Px s = p;
         if (OPT && C.d2) {
-            bool go = C.max_iter > 3;
-            for (int n = 1; n <= 3 && go; n++) {
-                s = step_full(s, C);
+            for (int n = 1; n <= min(3, C.max_iter - 1); n++) {
+                step_full(s, C);
                 if (n == 1) s.dzndz = cx(1., 0.);
                 std_opt_take<OPT>(s.o, C, n, s.zn);
-                go = StdMandel<OPT>::stop(s, C) < 0;
+                if (StdMandel<OPT>::stop(s, C) >= 0) break;
+                s.n = n;
+                p = s;
             }
-            s.n = 3;
-            if (go) p = s;
             return;
         }
         bool ok = dfac_ok(p.c) && C.max_iter > 2;
@@ -372,7 +389,7 @@ struct StdBS {
     static __device__ __forceinline__ int stop(const Px &p, const CalcDev &C) {
         return fsg_escaped(C, cx(p.X, p.Y)) ? 1 : -1;
     }
-    static __device__ __noinline__ Px step_full(Px p, const CalcDev &C) {
+    static __device__ __forceinline__ void step_full(Px &p, const CalcDev &C) {
         const int flavor = C.flavor;
         const double X = p.X, Y = p.Y, a = p.a, b = p.b;
         const double dXdA = p.Xa, dXdB = p.Xb, dYdA = p.Ya, dYdB = p.Yb;
@@ -416,12 +433,15 @@ struct StdBS {
             nYb = 2. * (fabs(X) * sgn(Y) * dYdB + sgn(X) * dXdB * fabs(Y)) - 1.;
         }
         p.X = nX; p.Y = nY; p.Xa = nXa; p.Xb = nXb; p.Ya = nYa; p.Yb = nYb;
-        return p;
     }
     // With X and Y in the range of the integer products and every derivative
     // there or 0 (flavors 4 and 5 keep dX/da = dY/da = 0): the products by
     // +-1 change signs, those by 2 exponents, and each remaining product and
     // sum rounds as in step_full.
+    static __device__ __forceinline__ bool in_range(const Px &p, const CalcDev &) {
+        return dfac_ok(p.X) & dfac_ok(p.Y) & dfac_ok0(p.Xa) & dfac_ok0(p.Xb) & dfac_ok0(p.Ya)
+               & dfac_ok0(p.Yb);
+    }
     static __device__ __forceinline__ void step(Px &p, const CalcDev &C) {
         const int flavor = C.flavor;
         bool ok = dfac_ok(p.X) & dfac_ok(p.Y) & dfac_ok0(p.Xa) & dfac_ok0(p.Xb)
@@ -453,14 +473,13 @@ struct StdBS {
         if (ok) {
             p.X = nX; p.Y = nY; p.Xa = xa; p.Xb = xb; p.Ya = ya; p.Yb = yb;
         } else {
-            p = step_full(p, C);
+            p = std_step_full<StdBS<OPT>>(p, C);
         }
     }
     static __device__ __forceinline__ void start(Px &p, const CalcDev &C) {
         // n = 1: X = a, Y = -b from zeros, in the plain form (one step's
         // operations for 32 pixels)
-        Px s = p;
-        s = step_full(s, C);
+        Px s = std_step_full<StdBS<OPT>>(p, C);
         std_opt_take<OPT>(s.o, C, 1, cx(s.X, s.Y));
         s.n = 1;
         if (C.max_iter > 1 && stop(s, C) < 0) p = s;
@@ -469,6 +488,7 @@ struct StdBS {
     // 5 dY/db; the partners are X and Y and the derivatives by one coordinate.
     // Every component is own X' +- pr Y' with X' = +-X or +-2 X, Y' likewise.
     static constexpr bool kCoop = !OPT;
+    static constexpr bool kPlain = true;
     static __device__ __forceinline__ double coop_get(const Px &p, int role) {
         return role == 0 ? p.X : role == 1 ? p.Y : role == 2 ? p.Xa : role == 3 ? p.Xb
                : role == 4 ? p.Ya : p.Yb;
@@ -510,13 +530,30 @@ struct StdBS {
         return L.add ? w : u;
     }
     static __device__ __forceinline__ double coop_full(double own, double pr, double x, double y,
-                                                       const Px &p, const CalcDev &C, int role, int) {
-        Px q = p;
-        q.X = x; q.Y = y;
-        // one of the two derivative pairs, in both places
-        q.Xa = q.Xb = role < 4 ? own : pr;
-        q.Ya = q.Yb = role < 4 ? pr : own;
-        return coop_get(step_full(q, C), role);
+                                                       const Px &, const CoopLane &L, const CalcDev &C,
+                                                       int role, int) {
+        const int flavor = C.flavor;
+        const bool ship = flavor == 1 || flavor == 5, fold = flavor >= 4;
+        // coop_fast by the multiplies, in one form for every role, the signs of zeros
+        // and sgn(0) = 1 as in step_full (which took all six components in every
+        // lane: flavor 3, 49 x 51 with a row on the axis, 1.45 -> 0.55 ms)
+        const unsigned sx = d_hi(x) & 0x80000000u, sy = d_hi(y) & 0x80000000u;
+        const unsigned nx = d_lt0(x) ? 0x80000000u : 0u, ny = d_lt0(y) ? 0x80000000u : 0u;
+        const unsigned f1 = role < 4 ? 0u : ship ? sx ^ ny : flavor == 2 ? ny : 0u;
+        const unsigned f2 = role < 4 ? L.neg ^ (flavor == 3 ? sy : 0u) : ship ? sy ^ nx : flavor == 2 ? sy : 0u;
+        double fx = d_flip(x, f1);
+        if (role == 1 && !ship) fx = 2. * x;
+        const double s = own * fx;
+        double u = s + pr * d_flip(y, f2);
+        if (role == 1) u = ship ? fabs(s) : flavor == 2 ? d_flip(s, sy) : s;
+        if (role > 1 || (role == 1 && ship)) u = 2. * u;
+        if (fold) {
+            const double q = x * x - y * y;
+            if ((role & 6) == 2) u = sgn(q) * u;
+            if (role == 0) u = fabs(u);
+        }
+        const double w = u + L.g;
+        return L.add ? w : u;
     }
     static __device__ __forceinline__ bool coop_near(double, double, double x, double y,
                                                      const CalcDev &C, int) {
@@ -600,9 +637,38 @@ __device__ __forceinline__ void std_coop(const WorkDev &W, const CalcDev &C, con
         bool ok = true;
         double next = Mdl::coop_fast(own, pr, x, y, L, C, base, role, ok);
         ok = ok & dfac_ok(cx(x, y)) & dfac_ok0(own) & dfac_ok0(pr);
-        if (have && !ok) next = Mdl::coop_full(own, pr, x, y, p, C, role, n);
+        if (have && !ok) next = Mdl::coop_full(own, pr, x, y, p, L, C, role, n);
         if (have) own = next;
     }
+}
+
+// Up to FSG_STD_CHUNK steps of a pixel by the multiplies; its stop reason, -1 to
+// go on.  Pixels on an axis and chaotic ones have zero factors or overflowing
+// derivatives at every step up to max_iter, and an image's last pixels are
+// such.  A warp pays for each form that one of its lanes takes, so while a lane
+// is out of the integer products' range all take the multiplies.  Out of line:
+// the loop keeps its registers and its instructions.  To 1000 iterations, with a
+// row on the axis, Burning Ship flavor 2, 201 x 203: 1.16 ms, 1.84 with both forms
+// taken, 1.40 with the multiplies alone; flavor 3 with the orbit point, 49 x 51:
+// 1.10, 1.88, 1.20 ms; power 2 with d2zndc2 and the orbit point, 49 x 51: 2.12,
+// 3.39, 2.64 ms (without the row: 1.13, 1.12, 2.14).  The power-2 loop without
+// options has no image that this helps (its tail runs in std_coop).
+template <class Mdl, bool OPT>
+static __device__ __noinline__ int std_plain_chunk(typename Mdl::Px &p, const CalcDev &C) {
+    typename Mdl::Px q = p;
+    int reason = -1;
+    for (int k = 0; k < FSG_STD_CHUNK && reason < 0; k++) {
+        q.n += 1;
+        reason = 0;
+        if (q.n < C.max_iter) {
+            Mdl::step_full(q, C);
+            std_after_step<OPT>(q, C);
+            reason = Mdl::stop(q, C);
+        }
+        std_opt_take<OPT>(q.o, C, q.n, std_z<OPT>(q));
+    }
+    p = q;
+    return reason;
 }
 
 // The loop (core.py:2935-3056).  Pixels reach a lane in three stages:
@@ -620,7 +686,7 @@ __device__ __forceinline__ void std_coop(const WorkDev &W, const CalcDev &C, con
 // The interruption flag is polled at claims and every FSG_STD_CANCEL chunks
 // (numba_cycles, core.py:2959-2960); it drops the waiting pixels.
 template <class Mdl, bool OPT>
-__global__ void __launch_bounds__(256) k_std(WorkDev W, CalcDev C) {
+__global__ void __launch_bounds__(256, OPT ? 2 : 1) k_std(WorkDev W, CalcDev C) {
     typedef typename Mdl::Px Px;
     __shared__ long long s_start[FSG_MAX_TILES_PER_LAUNCH + 1];
     __shared__ __align__(16) unsigned char s_raw[256 * sizeof(Px)];
@@ -640,8 +706,27 @@ __global__ void __launch_bounds__(256) k_std(WorkDev W, CalcDev C) {
     const int nwarps = (int)blockDim.x >> 5;
     bool alone = true;                 // the warp runs apart from its block
     bool told = false;
+    auto leave = [&](int reason) {
+        const TileDev &T = W.tiles[p.t];
+        Mdl::store(p, T, C);
+        T.stop_iter[p.ip] = p.n; T.stop_reason[p.ip] = (signed char)reason;
+        it_sum += (unsigned long long)p.n; fsg_account(W, (unsigned long long)p.n);
+        steps += (unsigned long long)(p.n - 1);
+        have = false;
+    };
     for (int chunk = 1;; chunk++) {
-        for (int k = 0; k < FSG_STD_CHUNK; k++) {
+        bool plain = false;
+        if constexpr (Mdl::kPlain) {
+            plain = __any_sync(0xffffffffu, have && !Mdl::in_range(p, C));
+            if (plain) {
+                Px q = p;
+                const int reason = have ? std_plain_chunk<Mdl, OPT>(q, C) : -1;
+                p = q;
+                if (reason >= 0) leave(reason);
+                __syncwarp();
+            }
+        }
+        for (int k = plain ? FSG_STD_CHUNK : 0; k < FSG_STD_CHUNK; k++) {
             if (k % FSG_STD_REFILL == 0 && (more || q_n > 0)) {
                 unsigned idle = __ballot_sync(0xffffffffu, !have);
                 while (idle != 0u && (more || q_n > 0)) {
@@ -677,14 +762,7 @@ __global__ void __launch_bounds__(256) k_std(WorkDev W, CalcDev C) {
                     reason = Mdl::stop(p, C);
                 }
                 std_opt_take<OPT>(p.o, C, p.n, std_z<OPT>(p));
-                if (reason >= 0) {
-                    const TileDev &T = W.tiles[p.t];
-                    Mdl::store(p, T, C);
-                    T.stop_iter[p.ip] = p.n; T.stop_reason[p.ip] = (signed char)reason;
-                    it_sum += (unsigned long long)p.n; fsg_account(W, (unsigned long long)p.n);
-                    steps += (unsigned long long)(p.n - 1);
-                    have = false;
-                }
+                if (reason >= 0) leave(reason);
             }
             __syncwarp();
         }
