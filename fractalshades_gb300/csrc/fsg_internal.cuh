@@ -383,10 +383,14 @@ inline int fsg_auto_grid(K kernel, int grid, int block, long long total, size_t 
 
 // Threads per CTA of an FP64 perturbation kernel where the caller leaves it open:
 // 256, or 64 for an image that the SMs hold all at once -- in CTAs of 256 some
-// SMs then hold one more CTA than others and finish that much later.
+// SMs then hold one more CTA than others and finish that much later.  Under a
+// limit on the CTAs of an SM (grid < 0) 256: a CTA of 64 would leave the SM a
+// quarter of the threads that the limit allows (200 x 200 pixels of the seahorse
+// view at one CTA an SM: 8.6 ms so, 6.0 with 256).
 template <class K>
-inline int fsg_fp64_block(K kernel, int block, long long total, size_t smem) {
+inline int fsg_fp64_block(K kernel, int grid, int block, long long total, size_t smem) {
     if (block > 0) return block;
+    if (grid < 0) return 256;
     const long long fit = 256LL * fsg_auto_grid(kernel, 0, 256, 1LL << 40, smem);
     return total <= fit ? 64 : 256;
 }

@@ -555,13 +555,13 @@ static void launch_m2(const WorkDev &W, const CalcDev &C, int grid, int block, c
         const long long two = 256LL * fsg_auto_grid(k_perturb_m2<XR, MN, ORB>, 0, 256, 1LL << 40, sm);
         if (!C.interior && total > two) {
             const size_t acc = 4 * sizeof(unsigned long long);      // per thread
-            const int b = fsg_fp64_block(k_perturb_m2_xr_dense, block, total, sm + 256 * acc);
+            const int b = fsg_fp64_block(k_perturb_m2_xr_dense, grid, block, total, sm + 256 * acc);
             const size_t smd = sm + acc * (size_t)b;
             k_perturb_m2_xr_dense<<<fsg_auto_grid(k_perturb_m2_xr_dense, grid, b, total, smd), b, smd, s>>>(W, C);
             return;
         }
     }
-    block = fsg_fp64_block(k_perturb_m2<XR, MN, ORB>, block, total, sm);
+    block = fsg_fp64_block(k_perturb_m2<XR, MN, ORB>, grid, block, total, sm);
     k_perturb_m2<XR, MN, ORB><<<fsg_auto_grid(k_perturb_m2<XR, MN, ORB>, grid, block, total, sm), block, sm,
                                 s>>>(W, C);
 }

@@ -13,7 +13,7 @@ template <class T, int FL, bool AXIS>
 static void launch_bs(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s) {
     const size_t acc = 4 * sizeof(unsigned long long);      // per thread
     size_t sm = fsg_starts_smem(W);
-    block = fsg_fp64_block(k_perturb_bs<T, FL, AXIS, false>, block, W.total - W.base, sm + 256 * acc);
+    block = fsg_fp64_block(k_perturb_bs<T, FL, AXIS, false>, grid, block, W.total - W.base, sm + 256 * acc);
     sm += acc * (size_t)block;
     k_perturb_bs<T, FL, AXIS, false><<<fsg_auto_grid(k_perturb_bs<T, FL, AXIS, false>, grid, block, W.total - W.base, sm),
                           block, sm, s>>>(W, C);

@@ -864,9 +864,10 @@ __global__ void __launch_bounds__(256) k_std_epilogue(WorkDev W, CalcDev C) {
     }
 }
 
-// block 0: chosen by the size.  Up to FSG_STD_FEW_PX pixels per SM eight lanes a
-// pixel (no budget, whose claims end early); below one 256-thread CTA per SM
-// CTAs of 64, so that the warps spread over the SMs.
+// block 0: chosen by the size, CTAs of 256 under a limit on the CTAs of an SM
+// (grid < 0).  Up to FSG_STD_FEW_PX pixels per SM eight lanes a pixel (no
+// budget, whose claims end early); below one 256-thread CTA per SM CTAs of 64, so
+// that the warps spread over the SMs.
 #define FSG_STD_FEW_PX 64
 template <class Mdl, bool OPT>
 static void launch_k_std(const WorkDev &W, const CalcDev &C, int grid, int block, cudaStream_t s) {
@@ -874,13 +875,13 @@ static void launch_k_std(const WorkDev &W, const CalcDev &C, int grid, int block
     if (block == 0) {
         const long long sms = fsg_auto_grid(k_std<Mdl, OPT>, -1, 256, 1LL << 40);   // one CTA per SM
         if constexpr (Mdl::kCoop) {
-            if (total <= FSG_STD_FEW_PX * sms && W.budget == 0 && W.order == nullptr) {
+            if (grid == 0 && total <= FSG_STD_FEW_PX * sms && W.budget == 0 && W.order == nullptr) {
                 const int per = FSG_STD_FEW_BLOCK / 8;
                 k_std_few<Mdl><<<(unsigned)((total + per - 1) / per), FSG_STD_FEW_BLOCK, 0, s>>>(W, C);
                 return;
             }
         }
-        block = total < 256 * sms ? 64 : 256;
+        block = grid == 0 && total < 256 * sms ? 64 : 256;
     }
     k_std<Mdl, OPT><<<fsg_auto_grid(k_std<Mdl, OPT>, grid, block, total), block, 0, s>>>(W, C);
 }

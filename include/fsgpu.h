@@ -127,9 +127,13 @@ typedef struct {
     int32_t block;            /* launch shape (chosen by the autotuner,
                                  fractalshades_gb300/tune.py): threads per
                                  CTA, 0 = the launcher's choice (128 for the
-                                 FE32 power-2 kernel; else 256, or 64 where the
-                                 FP64, XR64 and standard launchers see that the
-                                 SMs hold the whole image at once), else a
+                                 FE32 power-2 kernel; else 256, or, with no
+                                 ctas_per_sm: 64 where the FP64 and XR64
+                                 perturbation kernels hold the whole image on the
+                                 SMs at once; standard loops: 64 below 256 pixels
+                                 per SM, 128 with eight threads a pixel up to 64
+                                 pixels per SM, not for d2zndc2, orbit points,
+                                 the power-n model or a budget), else a
                                  multiple of 32 up to the kernel's bound (256;
                                  128 for the FE32 power-2 kernel)             */
     int32_t ctas_per_sm;      /* resident CTAs per SM of the persistent grid,
@@ -145,7 +149,9 @@ typedef struct {
                                  call returns FSG_BUDGET -- submit those pixels
                                  again to finish.  No counterpart in the
                                  reference (it runs a tile to its end)         */
-    int32_t claim_order;      /* FSG_ORDER_PIXELS (0): pixels claimed in order;
+    int32_t claim_order;      /* FSG_ORDER_PIXELS (0): pixels claimed in order
+                                 (perturbation: the 8 x 4 blocks of a rectangle,
+                                 row by row in a block and from block to block);
                                  FSG_ORDER_LONGEST (1): a perturbation launch of
                                  2^18 pixels or more claims them longest first
                                  (see fsg_perturb_tiles).  Outputs are the same;
