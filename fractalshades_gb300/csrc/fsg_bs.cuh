@@ -1197,10 +1197,12 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
                 };
                 fetch();
                 const bool bla_on = C.bla && R.bla_len > 0;
-                // X_0 = Y_0 = 0 and no BLA attempt there: after a rebase the step
-                // at w = 0 follows at once
+                // X_0 = Y_0 = 0 and no BLA attempt there (the loop's own condition):
+                // after a rebase the step at w = 0 follows at once.  200^2 pixels of
+                // a period-12 nucleus to 3000 iterations: 1.41 ms, 1.61 without
                 const bool crit0 = FL == 1 && (__ldg(&R.bs_at[0]).x & 4)
-                                   && !(bla_on && (1 << FSG_STG_COMPRESSED) < R.first_invalid);
+                                   && !(bla_on && (1 << FSG_STG_COMPRESSED) < R.first_invalid
+                                        && bla_possible(R, 0));
                 for (;;) {
                     if (bla_on && (w & 7) == 0 &&
                         (1 << FSG_STG_COMPRESSED) < R.first_invalid - w && bla_possible(R, w)) {
