@@ -1186,14 +1186,22 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
             // (0), a BLA step was taken (1), the step at w has to run in fr (2) or
             // the tests at w have to (3); the fr values are current on return.
             auto frame_run = [&]() -> int {
-                // the records of w, read together as soon as w is known
+                // the records of w, read together as soon as w is known; flavor 5
+                // reads the Hessian's where it uses it: its views leave the frame
+                // form for fr steps often, and need it at fewer points (100^2
+                // pixels of a period-17 nucleus to 3000 iterations: 8.80 ms with
+                // all three, 8.50 so)
+                constexpr bool HM_LATE = FL == 5;
                 int4 fz;
                 float4 fa, Hm = make_float4(0.f, 0.f, 0.f, 0.f);
                 auto fetch = [&]() {
                     const int4 *at = R.bs_at + 3 * (size_t)w;
                     fz = __ldg(at);
                     fa = __ldg((const float4 *)at + 1);
-                    if (hess) Hm = __ldg((const float4 *)at + 2);
+                    if (hess && !HM_LATE) Hm = __ldg((const float4 *)at + 2);
+                };
+                auto fetch_late = [&]() {
+                    if (hess) Hm = __ldg((const float4 *)(R.bs_at + 3 * (size_t)w) + 2);
                 };
                 fetch();
                 const bool bla_on = C.bla && R.bla_len > 0;
@@ -1216,6 +1224,10 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
                         }
                     }
                     if (!(fz.x & 5)) { frame_out(Fm, xn, yn, h); return 2; }
+                    if constexpr (HM_LATE) {
+                        if (dyn) Hm = make_float4(0.f, 0.f, 0.f, 0.f);
+                        else fetch_late();
+                    }
                     if (fz.x & 4) {
                         if (FL == 1 && dyn) bs_frame_zero1(hess, Fm);
                         else bs_frame_step_zero(flavor, hess, Fm, Hm, fz.y, dyn);
@@ -1261,6 +1273,7 @@ FSG_DEV int pixel_bs(const TileDev &T_, const CalcDev &C, long long ip, unsigned
                     if (res == 1) { stop = 1; frame_out(Fm, xn, yn, h); return 0; }
                     if (res == 2) {
                         // rebase where X + xn, Y + yn round to the deltas: they stay
+                        if constexpr (HM_LATE) fetch_late();
                         if (hess) frame_add_hess(Fm, Hm, fz.y);
                         if (!divr) dyn = true;
                         const bool there = w == 0;
