@@ -12,7 +12,9 @@ dzndc distance estimate.  One step = one launch over the whole image.
 
     python bench.py [--steps K] [--warmup W] [--gpus N] [--impl ours|reference]
 
-Prints one JSON line.  With torchrun (N > 1) every rank renders its own
+Prints one JSON line of a few kilobytes; what the serving stream and the other
+configurations measured in full goes to standard error, a JSON line too, with
+their times in the printed one.  With torchrun (N > 1) every rank renders its own
 replica of the image (the pixels are independent) and rank 0 prints.
 """
 import argparse
@@ -33,6 +35,31 @@ METRIC = "pixel-iter/s at 1e-300 zoom, FP32+exp vs FP64 path; p50/p99 tile laten
 FLOPS_FULL = 35      # M2 perturbation step with dzndc (zn 17 + dzndc 18)
 FLOPS_BLA = 23       # M2 BLA step with dzndc (17 + 6)
 LIN = np.array([[1., -0.], [0., 1.]])
+
+
+def short_line(line):
+    """The printed line: ``serving`` and ``supplementary`` (some 20 kB of tables,
+    more than a reader of the last lines of a log keeps) reduced to the
+    latencies and rates per order and to each configuration's times."""
+    out = dict(line)
+    if line.get("serving"):
+        out["serving"] = {
+            order: {"pixel_iter_per_s": r["pixel_iter_per_s"], "p50_ms": r["latency_ms"]["p50"],
+                    "p99_ms": r["latency_ms"]["p99"]}
+            for order, r in line["serving"].items() if isinstance(r, dict) and "latency_ms" in r}
+    if line.get("supplementary"):
+        times = {}
+
+        def walk(path, v):
+            if isinstance(v, dict):
+                for k, x in v.items():
+                    walk(path + [k], x)
+            elif path[-1] in ("kernel_ms", "s") or path[-1].endswith("_s"):
+                if isinstance(v, (int, float)) and not {"vs_oracle", "vs_exact"} & set(path):
+                    times[".".join(path)] = float("%.5g" % v)
+        walk([], line["supplementary"])
+        out["supplementary"] = times
+    return out
 
 
 def parse():
@@ -1156,7 +1183,8 @@ def run_ours(args):
                                        "path": "page-locked arrays reused per size, "
                                                "written in place"}},
     }
-    print(json.dumps(line), flush=True)
+    print(json.dumps({"serving": serving, "supplementary": supp}), file=sys.stderr, flush=True)
+    print(json.dumps(short_line(line)), flush=True)
     if dist:
         dist.barrier()
     return 0
