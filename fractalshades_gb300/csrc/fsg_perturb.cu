@@ -239,7 +239,7 @@ __device__ __forceinline__ bool dz_below(double2 Z, double2 z, int e) {
 
 // The power-2 loop, both delta forms.  The reference's operations with their
 // bits, arranged for GB300's pipes (an FP64 warp instruction holds its pipe for
-// 64 clocks and more, of which a step had 31): products on the integer pipes
+// some 80 clocks, of which a step had 31): products on the integer pipes
 // (fsg_soft.cuh), sums left out where an operand is below half an ulp of the
 // other, the escape test and the BLA radii on upper words.  XR: every value is a
 // mantissa and an exponent of its own frame; the bits of a value do not depend
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(256) k_perturb_m2(WorkDev W, CalcDev C) {
 }
 
 // The Xrange power-2 loop at three CTAs of 256 an SM (80 registers, with spills)
-// instead of two (123): the latency of its chains bounds it.  513 x 511 pixels of
+// instead of two (121): the latency of its chains bounds it.  513 x 511 pixels of
 // the period-2562 nucleus take 10.0 ms so and 10.8 with two, 300 x 300 (one wave of
 // three, two of two) 22 % less.  The statistics are 32-bit per pixel and summed in
 // shared memory, where 64-bit sums would hold 8 registers in the loop (10.3 ms).

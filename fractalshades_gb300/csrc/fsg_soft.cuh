@@ -1,11 +1,13 @@
 // fsg_soft.cuh -- products of doubles on the integer pipes, bit for bit.
 //
-// An SM of GB300 issues 1.63 FP64 thread-operations a clock, 62 of 32-bit
-// logic, shifts or adds and 26 of 32 x 32 + 64 -> 64-bit multiply-adds (all
-// measured).  A correctly rounded 53 x 53-bit product is four of those
+// An SM of GB300 issues 1.6 FP64 thread-operations a clock, 61 of 32-bit
+// logic or shifts and 26 of 32 x 32 + 64 -> 64-bit multiply-adds (measured on
+// eight independent chains a thread, 4 CTAs of 256 an SM: 0.503e12, 19.1e12 and
+// 8.2e12 a second at 2070 MHz).  A correctly rounded 53 x 53-bit product is four of those
 // multiply-adds and about a dozen others, so a loop that multiplies here and
 // adds on the FP64 pipe keeps both busy: eight chains of products alone run at
-// 1.6 products per SM and clock by DMUL and at 3.5 with five of the eight here.
+// 1.6 products per SM and clock by DMUL, at 4.2 with five of the eight here and at
+// 3.0 with all of them here (0.503, 1.32 and 0.95e12 a second).
 //
 // dfac is a factor: the sign and exponent fields of a double and its 53-bit
 // mantissa shifted up by 6 (two 32-bit words, the upper one below 2^27, so that
@@ -262,17 +264,12 @@ FSG_DEV void frame_renorm(xc &a, bool &ok) {
     a.e += k;
 }
 
-// xr_mul and xr_mul_s by the integer products
+// xr_mul by the integer products
 FSG_DEV xc xs_mul(xc a, xc b) {
     double2 m = cmul_soft(xm(a), xm(b));
     int e = (int)((unsigned)a.e + (unsigned)b.e);
     if (xr_need_renorm_c(m)) return xr_normalize_c(m, e);
     return xc_make(m.x, m.y, e);
-}
-FSG_DEV xc xs_mul_s(double2 s, xc b) {
-    double2 m = cmul_soft(s, xm(b));
-    if (xr_need_renorm_c(m)) return xr_normalize_c(m, b.e);
-    return xc_make(m.x, m.y, b.e);
 }
 
 // ---------------------------------------------------------------------------
