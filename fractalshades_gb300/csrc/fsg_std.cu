@@ -534,7 +534,8 @@ struct StdBS {
                                                        int role, int) {
         const int flavor = C.flavor;
         const bool ship = flavor == 1 || flavor == 5, fold = flavor >= 4;
-        // coop_fast by the multiplies, in one form for every role, the signs of zeros
+        // coop_fast by the multiplies (nowhere ahead of their branch: computed at every
+        // step they cost as much again), in one form for every role, the signs of zeros
         // and sgn(0) = 1 as in step_full (which took all six components in every
         // lane: flavor 3, 49 x 51 with a row on the axis, 1.45 -> 0.55 ms)
         const unsigned sx = d_hi(x) & 0x80000000u, sy = d_hi(y) & 0x80000000u;
@@ -542,18 +543,17 @@ struct StdBS {
         const unsigned f1 = role < 4 ? 0u : ship ? sx ^ ny : flavor == 2 ? ny : 0u;
         const unsigned f2 = role < 4 ? L.neg ^ (flavor == 3 ? sy : 0u) : ship ? sy ^ nx : flavor == 2 ? sy : 0u;
         double fx = d_flip(x, f1);
-        if (role == 1 && !ship) fx = 2. * x;
-        const double s = own * fx;
-        double u = s + pr * d_flip(y, f2);
+        if (role == 1 && !ship) fx = d_mul_here(2., x);
+        const double s = d_mul_here(own, fx);
+        double u = d_add_here(s, d_mul_here(pr, d_flip(y, f2)));
         if (role == 1) u = ship ? fabs(s) : flavor == 2 ? d_flip(s, sy) : s;
-        if (role > 1 || (role == 1 && ship)) u = 2. * u;
+        if (role > 1 || (role == 1 && ship)) u = d_mul_here(2., u);
         if (fold) {
-            const double q = x * x - y * y;
-            if ((role & 6) == 2) u = sgn(q) * u;
+            const double q = d_add_here(d_mul_here(x, x), -d_mul_here(y, y));
+            if ((role & 6) == 2 && d_lt0(q)) u = -u;
             if (role == 0) u = fabs(u);
         }
-        const double w = u + L.g;
-        return L.add ? w : u;
+        return L.add ? d_add_here(u, L.g) : u;
     }
     static __device__ __forceinline__ bool coop_near(double, double, double x, double y,
                                                      const CalcDev &C, int) {
@@ -699,6 +699,7 @@ __global__ void __launch_bounds__(256, OPT ? 2 : 1) k_std(WorkDev W, CalcDev C) 
     Px *queue = s_px + (threadIdx.x & ~31);
     int q_n = 0;                       // pixels waiting
     bool more = true;                  // pixels may be left to claim
+    bool first = true;                 // the warp's first claim
     long long last = 0;
     Px p;
     Mdl::init(p, C, cx(0., 0.));
@@ -732,7 +733,8 @@ __global__ void __launch_bounds__(256, OPT ? 2 : 1) k_std(WorkDev W, CalcDev C) 
                 while (idle != 0u && (more || q_n > 0)) {
                     if (q_n == 0) {
                         Px s;
-                        q_n = fsg_claim_warp(W, s_start, __popc(idle), last, s.t, s.ip);
+                        q_n = fsg_claim_warp(W, s_start, __popc(idle), first, last, s.t, s.ip);
+                        first = false;
                         more = q_n > 0;
                         if (lane < q_n) {
                             Mdl::init(s, C, std_c(W.tiles[s.t], s.ip));
